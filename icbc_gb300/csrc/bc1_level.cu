@@ -17,21 +17,41 @@ namespace icbc_gpu {
 
 // ------------------------------------------------------------- kernels --
 
+// How many of n blocks a worker (a warp of 32 lanes, or a CTA) takes at a
+// time when `workers` share them: as few as the rounds they need anyway allow,
+// at most `most`.  A last round that is nearly empty costs as much as a full
+// one, and an image too small for 32 blocks a warp leaves most SMs without a
+// warp while the others run long ones (the cluster search spreads a warp's
+// blocks over its 32 lanes however many they are).  Against 32 blocks a warp
+// always, in us: level 8 at 64 x 64 187 -> 48, 512 x 512 194 -> 116, 2048 x
+// 2048 (the 16-warp CTAs' last round) 1018 -> 826, 4096 x 4096 3342 -> 3114;
+// with a weight plane 1000 x 600 431 -> 237; 40,000 float blocks 303 -> 155.
+// A warp takes at least `least` blocks: below level 4, where the search is a
+// small part of a block's work, warps with few blocks only add lanes without
+// one (level 3 at 1024 x 1024: 45 us with 16, 51 with 1; level 7 at 64 x 64:
+// 79 with 16, 48 with 1).
+__host__ __device__ constexpr int balanced_share(int64_t n, int64_t workers, int most, int least) {
+    const int64_t rounds = (n + workers * most - 1) / (workers * most);
+    const int64_t share = rounds < 1 ? 1 : (n + workers * rounds - 1) / (workers * rounds);
+    return (int)(share < least ? least : share);
+}
+__host__ __device__ constexpr int least_per_warp(int level) { return level >= 4 ? 1 : 16; }
+
 // With DEFER (level 9 only) refinement is left to k_refine: the kernel
 // records each block's starting error and whether refinement applies.
 template <int L, bool DEFER>
 __global__ void __launch_bounds__(kWarpsPerCta * 32) k_encode_blocks(const GlobalTables *G, BlocksSrc s, EncodeParams p,
-                                                                     uint2 *out, float *errors, int64_t n,
+                                                                     uint2 *out, float *errors, int64_t n, int per_warp,
                                                                      RefineSlot *st) {
     extern __shared__ __align__(16) unsigned char smem[];
     SharedTables &T = *reinterpret_cast<SharedTables *>(smem);
     stage_tables(T, G);
     const WarpCtx w = warp_ctx<L>(smem, T, G, p.decoder);
-    const int64_t groups = (n + 31) / 32;
+    const int64_t groups = (n + per_warp - 1) / per_warp;
     for (int64_t g = (int64_t)blockIdx.x * kWarpsPerCta + (threadIdx.x >> 5); g < groups;
          g += (int64_t)gridDim.x * kWarpsPerCta) {
-        const int64_t base = g * 32;
-        const int nb = (int)(n - base < 32 ? n - base : 32);
+        const int64_t base = g * per_warp;
+        const int nb = (int)(n - base < per_warp ? n - base : per_warp);
         __syncwarp();
         load_float_blocks(s, base, nb, w.in, w.lane);
         __syncwarp();
@@ -56,16 +76,16 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32) k_encode_blocks(const Globa
 
 template <int L, bool DEFER>
 __global__ void __launch_bounds__(kWarpsPerCta * 32) k_encode_image(const GlobalTables *G, ImageDesc d, EncodeParams p,
-                                                                    RefineSlot *st) {
+                                                                    int per_warp, RefineSlot *st) {
     extern __shared__ __align__(16) unsigned char smem[];
     SharedTables &T = *reinterpret_cast<SharedTables *>(smem);
     stage_tables(T, G);
     const WarpCtx w = warp_ctx<L>(smem, T, G, p.decoder);
-    const int64_t groups = (d.nblocks + 31) / 32;
+    const int64_t groups = (d.nblocks + per_warp - 1) / per_warp;
     for (int64_t g = (int64_t)blockIdx.x * kWarpsPerCta + (threadIdx.x >> 5); g < groups;
          g += (int64_t)gridDim.x * kWarpsPerCta) {
-        const int64_t b = g * 32 + w.lane;
-        const bool active = b < d.nblocks;
+        const int64_t b = g * per_warp + w.lane;
+        const bool active = w.lane < per_warp && b < d.nblocks;
         __syncwarp();
         if (active) load_image_block(d, b, w.in + w.lane * kInStride, T.lut255);
         __syncwarp();
@@ -91,17 +111,18 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32) k_encode_image(const Global
 // registers per thread, so four CTAs (16 warps) fit on an SM instead of three.
 template <int L, bool DEFER>
 __global__ void __launch_bounds__(kWarpsPerCta * 32, 4) k_encode_image_bytes(const GlobalTables *G, ImageDesc d,
-                                                                             EncodeParams p, RefineSlot *st) {
+                                                                             EncodeParams p, int per_warp,
+                                                                             RefineSlot *st) {
     extern __shared__ __align__(16) unsigned char smem[];
     SharedTables &T = *reinterpret_cast<SharedTables *>(smem);
     stage_tables(T, G);
     const WarpCtx w = warp_ctx_byte_rows(smem, T, G, p.decoder);
     const ByteRow row = byte_row(w, d.weight_mode == ICBC_GPU_WEIGHTS_ALPHA);
-    const int64_t groups = (d.nblocks + 31) / 32;
+    const int64_t groups = (d.nblocks + per_warp - 1) / per_warp;
     for (int64_t g = (int64_t)blockIdx.x * kWarpsPerCta + (threadIdx.x >> 5); g < groups;
          g += (int64_t)gridDim.x * kWarpsPerCta) {
-        const int64_t b = g * 32 + w.lane;
-        const bool active = b < d.nblocks;
+        const int64_t b = g * per_warp + w.lane;
+        const bool active = w.lane < per_warp && b < d.nblocks;
         __syncwarp();
         if (active) load_image_block_bytes(d, b, reinterpret_cast<uint32_t *>(w.in) + w.lane * kInWordsByte);
         __syncwarp();
@@ -185,7 +206,8 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32, 4) k_image_listed(const Glo
                                                                        EncodeParams p, const uint32_t *list,
                                                                        const unsigned int *listed, RefineSlot *st) {
     const int64_t n = *listed;
-    const int64_t groups = (n + 31) / 32;
+    const int per_warp = balanced_share(n, (int64_t)gridDim.x * kWarpsPerCta, 32, least_per_warp(L));
+    const int64_t groups = (n + per_warp - 1) / per_warp;
     if ((int64_t)blockIdx.x * kWarpsPerCta >= groups) return;  // the whole CTA has no work
     extern __shared__ __align__(16) unsigned char smem[];
     SharedTables &T = *reinterpret_cast<SharedTables *>(smem);
@@ -194,8 +216,8 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32, 4) k_image_listed(const Glo
     const ByteRow row = byte_row(w, d.weight_mode == ICBC_GPU_WEIGHTS_ALPHA);
     for (int64_t g = (int64_t)blockIdx.x * kWarpsPerCta + (threadIdx.x >> 5); g < groups;
          g += (int64_t)gridDim.x * kWarpsPerCta) {
-        const int64_t k = g * 32 + w.lane;
-        const bool active = k < n;
+        const int64_t k = g * per_warp + w.lane;
+        const bool active = w.lane < per_warp && k < n;
         const int64_t b = active ? (int64_t)list[k] : 0;
         __syncwarp();
         if (active) load_image_block_bytes(d, b, reinterpret_cast<uint32_t *>(w.in) + w.lane * kInWordsByte);
@@ -280,7 +302,8 @@ __global__ void __launch_bounds__(NW * 32, 512 / (NW * 32))
     k_image_listed_cta(const GlobalTables *G, ImageDesc d, EncodeParams p, const uint32_t *list,
                        const unsigned int *listed, RefineSlot *st) {
     const int64_t n = *listed;
-    const int64_t groups = (n + 32 * NW - 1) / (32 * NW);
+    const int per_cta = balanced_share(n, gridDim.x, 32 * NW, 1);
+    const int64_t groups = (n + per_cta - 1) / per_cta;
     if ((int64_t)blockIdx.x >= groups) return;  // the whole CTA has no work
     extern __shared__ __align__(16) unsigned char smem[];
     SharedTables &T = *reinterpret_cast<SharedTables *>(smem);
@@ -291,8 +314,8 @@ __global__ void __launch_bounds__(NW * 32, 512 / (NW * 32))
     uint32_t *in = reinterpret_cast<uint32_t *>(g.in);
     const ByteRow row = byte_row(w, d.weight_mode == ICBC_GPU_WEIGHTS_ALPHA);
     for (int64_t grp = blockIdx.x; grp < groups; grp += gridDim.x) {
-        const int64_t k = grp * (32 * NW) + threadIdx.x;
-        const bool active = k < n;
+        const int64_t k = grp * per_cta + threadIdx.x;
+        const bool active = (int)threadIdx.x < per_cta && k < n;
         const int64_t b = active ? (int64_t)list[k] : 0;
         __syncwarp();
         if (active) load_image_block_bytes(d, b, in + threadIdx.x * kInWordsByte);
@@ -414,27 +437,36 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32, 4)
 constexpr int L = ICBC_LEVEL;
 constexpr bool kCompact = Level<L>::cluster;
 
-// CTAs for n blocks, from the level's launch shape: every warp takes
-// groups_per_warp groups of 32 blocks; a persistent grid is exactly the
-// resident CTAs (from the occupancy API), each warp striding over the image,
-// otherwise there are enough CTAs for the work and the hardware balances
-// them (better when block costs vary, as they do from level 2 on).
+// CTAs for n blocks and the blocks a warp takes at a time.  An image of many
+// rounds takes the level's launch shape: every warp takes groups_per_warp
+// groups of 32 blocks; a persistent grid is exactly the resident CTAs (from
+// the occupancy API), each warp striding over the image, otherwise there are
+// enough CTAs for the work and the hardware balances them (better when block
+// costs vary, as they do from level 2 on).  From level 2 on, one of fewer than
+// kBalancedRounds rounds gives each warp one group of a balanced size.
+constexpr int kBalancedRounds = 8;
 template <class K>
-static int grid_for(K kernel, int64_t n, int sms, size_t smem, int &resident) {
+static int grid_for(K kernel, int64_t n, int sms, size_t smem, int &resident, int *per_warp = nullptr) {
     const LaunchShape shape = launch_shape(L);
+    if (!resident) {
+        int per_sm = 0;
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kWarpsPerCta * 32, smem) != cudaSuccess ||
+            per_sm < 1)
+            per_sm = 1;
+        resident = per_sm;
+    }
+    const int64_t cap = (int64_t)sms * resident;
+    if (per_warp) {
+        *per_warp = 32;
+        if (L >= 2 && n < cap * kWarpsPerCta * 32 * kBalancedRounds) {
+            *per_warp = balanced_share(n, cap * kWarpsPerCta, 32, least_per_warp(L));
+            return (int)((n + (int64_t)*per_warp * kWarpsPerCta - 1) / ((int64_t)*per_warp * kWarpsPerCta));
+        }
+    }
     const int64_t groups = (n + 31) / 32;
     const int64_t per_cta = (int64_t)kWarpsPerCta * shape.groups_per_warp;
     int64_t ctas = (groups + per_cta - 1) / per_cta;
     if (shape.persistent) {
-        if (!resident) {
-            int per_sm = 0;
-            if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kWarpsPerCta * 32, smem) !=
-                    cudaSuccess ||
-                per_sm < 1)
-                per_sm = 1;
-            resident = per_sm;
-        }
-        const int64_t cap = (int64_t)sms * resident;
         const int64_t all = (groups + kWarpsPerCta - 1) / kWarpsPerCta;
         ctas = all < cap ? all : cap;
     }
@@ -459,9 +491,10 @@ static cudaError_t run(Kernel kernel, size_t smem, int &resident, int64_t n, int
                        unsigned long long *ext_counter = nullptr) {
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    const int grid = grid_for(kernel, n, sms, smem, resident);
+    int per_warp = 32;
+    const int grid = grid_for(kernel, n, sms, smem, resident, &per_warp);
     if (!kDefer) {
-        launch(grid, smem, nullptr);
+        launch(grid, smem, per_warp, nullptr);
         return cudaGetLastError();
     }
     void *scratch = nullptr;
@@ -476,7 +509,7 @@ static cudaError_t run(Kernel kernel, size_t smem, int &resident, int64_t n, int
     }
     e = cudaMemsetAsync(counter, 0, sizeof(unsigned long long), stream);
     if (e == cudaSuccess) {
-        launch(grid, smem, st);
+        launch(grid, smem, per_warp, st);
         e = cudaGetLastError();
     }
     if (e == cudaSuccess) e = launch_refine(G, image, blocks, p, out, errors, st, n, counter, stream, sms);
@@ -572,7 +605,7 @@ static cudaError_t launch_image_compacted(const GlobalTables *G, const ImageDesc
     }
     if (e == cudaSuccess) {
         // Persistent over the list, whose length only the device knows.
-        const int per_cta = 32 * (cta_warps == 4 ? kWarpsPerCta : cta_warps);
+        const int per_cta = cta_warps == 4 ? kWarpsPerCta * least_per_warp(L) : 32 * cta_warps;
         const int64_t most = ((int64_t)d.nblocks + per_cta - 1) / per_cta;
         const int64_t cap = (int64_t)sms * *resident;
         const int grid = (int)(most < cap ? most : cap);
@@ -599,14 +632,14 @@ static cudaError_t launch_image(const GlobalTables *G, const ImageDesc &d, const
         if (use_byte_rows(d))
             return run(k_encode_image_bytes<L, kDefer>, smem_bytes_byte_rows(), g_resident_bytes, d.nblocks, sms,
                        stream,
-                       [&](int grid, size_t smem, RefineSlot *slots) {
-                           k_encode_image_bytes<L, kDefer><<<grid, kWarpsPerCta * 32, smem, stream>>>(G, d, p, slots);
+                       [&](int grid, size_t smem, int per_warp, RefineSlot *slots) {
+                           k_encode_image_bytes<L, kDefer><<<grid, kWarpsPerCta * 32, smem, stream>>>(G, d, p, per_warp, slots);
                        },
                        G, &d, nullptr, p, d.out, d.errors, ext_st, ext_counter);
     }
     return run(k_encode_image<L, kDefer>, smem_bytes(Level<L>::cluster), g_resident_image, d.nblocks, sms, stream,
-               [&](int grid, size_t smem, RefineSlot *slots) {
-                   k_encode_image<L, kDefer><<<grid, kWarpsPerCta * 32, smem, stream>>>(G, d, p, slots);
+               [&](int grid, size_t smem, int per_warp, RefineSlot *slots) {
+                   k_encode_image<L, kDefer><<<grid, kWarpsPerCta * 32, smem, stream>>>(G, d, p, per_warp, slots);
                },
                G, &d, nullptr, p, d.out, d.errors, ext_st, ext_counter);
 }
@@ -615,8 +648,8 @@ cudaError_t ICBC_CAT(launch_blocks_l, ICBC_LEVEL)(const GlobalTables *G, const B
                                                   void *out, float *errors, int64_t n, cudaStream_t stream, int sms) {
     uint2 *o = reinterpret_cast<uint2 *>(out);
     return run(k_encode_blocks<L, kDefer>, smem_bytes(Level<L>::cluster), g_resident_blocks, n, sms, stream,
-               [&](int grid, size_t smem, RefineSlot *st) {
-                   k_encode_blocks<L, kDefer><<<grid, kWarpsPerCta * 32, smem, stream>>>(G, s, p, o, errors, n, st);
+               [&](int grid, size_t smem, int per_warp, RefineSlot *st) {
+                   k_encode_blocks<L, kDefer><<<grid, kWarpsPerCta * 32, smem, stream>>>(G, s, p, o, errors, n, per_warp, st);
                },
                G, nullptr, &s, p, o, errors);
 }
