@@ -398,6 +398,18 @@ __device__ __forceinline__ uint32_t indices_generic(const Row &row, V3 cw, const
     return out;
 }
 
+// The endpoints step i of refine_endpoints, whose delta is (dr, dg, db), tries
+// from (r0, r1) (icbc.h:3614-3633).
+__device__ __forceinline__ void refine_candidate(int i, int dr, int dg, int db, const EncodeParams &p, uint32_t &r0,
+                                                 uint32_t &r1) {
+    if ((i >> 4) & 1) r0 = add565(r0, dr, dg, db);
+    else r1 = add565(r1, dr, dg, db);
+    if (!p.three_color_mode) {
+        if (r0 == r1) r1 = add565(r1, 0, 1, 0);
+        if (r0 < r1) { const uint32_t t = r0; r0 = r1; r1 = t; }
+    }
+}
+
 // refine_endpoints (icbc.h:3574-3651).  Indices of a step come from the
 // palette of the current best block, so they change only when a step is
 // accepted; the step's error uses the moved endpoints' palette.
@@ -408,15 +420,9 @@ __device__ __forceinline__ float refine(const WarpCtx &w, const Row &row, const 
     int last = 0;
     uint32_t base_idx = indices_generic(row, p.cw, palette_f(c0, c1, p.decoder, w.T->lut255, w.D));
     for (int i = 0; i < 256; i++) {
-        const int d = i & 15;
-        const int dr = c_deltas[d][0], dg = c_deltas[d][1], db = c_deltas[d][2];
+        const int8_t *d = c_deltas[i & 15];
         uint32_t r0 = c0, r1 = c1;
-        if ((i >> 4) & 1) r0 = add565(r0, dr, dg, db);
-        else r1 = add565(r1, dr, dg, db);
-        if (!p.three_color_mode) {
-            if (r0 == r1) r1 = add565(r1, 0, 1, 0);
-            if (r0 < r1) { const uint32_t t = r0; r0 = r1; r1 = t; }
-        }
+        refine_candidate(i, d[0], d[1], d[2], p, r0, r1);
         const PalF pr = palette_f(r0, r1, p.decoder, w.T->lut255, w.D);
         const float e = block_error(row, p.cw, pr, base_idx);
         if (e < best) {
@@ -480,15 +486,9 @@ __device__ __forceinline__ float block_error_pal(const Row &row, V3 cw, const Pa
 template <class Row>
 __device__ __forceinline__ bool refine_try(const WarpCtx &w, const float *lut, const Row &row, const EncodeParams &p,
                                            RefineLane &s, PalF &pr, bool &stop, float4 *pal = nullptr) {
-    const int d = s.i & 15;
-    const int dr = c_deltas[d][0], dg = c_deltas[d][1], db = c_deltas[d][2];
+    const int8_t *d = c_deltas[s.i & 15];
     uint32_t r0 = s.c0, r1 = s.c1;
-    if ((s.i >> 4) & 1) r0 = add565(r0, dr, dg, db);
-    else r1 = add565(r1, dr, dg, db);
-    if (!p.three_color_mode) {
-        if (r0 == r1) r1 = add565(r1, 0, 1, 0);
-        if (r0 < r1) { const uint32_t t = r0; r0 = r1; r1 = t; }
-    }
+    refine_candidate(s.i, d[0], d[1], d[2], p, r0, r1);
     pr = palette_f(r0, r1, p.decoder, lut, w.D);
     const float e = pal ? block_error_pal<4>(row, p.cw, pr, pal, s.base_idx) : block_error<4>(row, p.cw, pr, s.base_idx);
     const bool accept = e < s.best;

@@ -59,6 +59,18 @@ __device__ __forceinline__ void fetch_image_block(const ImageDesc &d, int64_t b,
     }
 }
 
+// Texel t of block b of an RGBA8 image and its weight, as floats (u8 -> float
+// is the exact table of i / 255.0f).
+__device__ __forceinline__ float4 load_image_texel(const ImageDesc &d, int64_t b, int t, const float *lut) {
+    const int bx = (int)(b % d.bw), by = (int)(b / d.bw);
+    const int x = min(4 * bx + (t & 3), d.width - 1), y = min(4 * by + (t >> 2), d.height - 1);
+    const uint32_t v = __ldg(reinterpret_cast<const uint32_t *>(d.rgba + (int64_t)y * d.pitch) + x);
+    float w = 1.0f;
+    if (d.weight_mode == 1) w = lut[v >> 24];
+    else if (d.weight_mode == 2) w = __ldg(d.weight_plane + (int64_t)y * d.weight_pitch + x);
+    return make_float4(lut[v & 255], lut[(v >> 8) & 255], lut[(v >> 16) & 255], w);
+}
+
 // One block of an RGBA8 image into this lane's float row.  u8 -> float is
 // the exact table of i / 255.0f.
 __device__ __forceinline__ void load_image_block(const ImageDesc &d, int64_t b, float *row, const float *lut) {

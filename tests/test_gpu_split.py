@@ -49,3 +49,14 @@ def test_cta_rounds(gpu_lib, level, bh):
     """Images of the 16-warp CTAs: the listed blocks just under and over whole rounds of 152 x 512."""
     img = synth.quality_sweep_image(4 * 512, 4 * bh, seed=bh)
     check(gpu_lib, img, level, 1, None)
+
+
+@pytest.mark.parametrize("n,decoders", ((1, (0, 1, 2, 3)), (700, (0, 1, 2, 3)), (97279, (1,)), (97281, (0,))))
+def test_refinement_counts(gpu_lib, n, decoders):
+    """A warp a block below one block for each of 152 x 640 lanes, a block a lane from there on."""
+    cols, w = synth.mixed_blocks(n, seed=n)
+    for dec in decoders:
+        for tc, tcb in ((True, True), (False, False)):
+            b, e = gpu_lib.compress_blocks(cols, w, 9, dec, (0.299, 0.587, 0.114), tc, tcb)
+            ob, oe = O.compress_blocks(cols, w, 9, dec, (0.299, 0.587, 0.114), tc, tcb, nthreads=16)
+            assert np.array_equal(b, ob) and np.array_equal(e.view(np.uint32), oe.view(np.uint32))
