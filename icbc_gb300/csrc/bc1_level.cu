@@ -537,13 +537,17 @@ static int listed_cta_warps() {
     return L >= 4 ? 16 : 4;
 }
 
-// The CTA size for an image of `nblocks` blocks: a CTA-wide pass takes
-// 32 * cta_warps listed blocks per CTA, so an image with fewer blocks than
-// two such rounds over every SM would run on a fraction of the SMs; it takes
-// 4-warp CTAs instead.
+// The CTA size for an image of `nblocks` blocks.  A CTA-wide pass shares the
+// blocks out evenly over the resident CTAs (balanced_share), so it pays from
+// few blocks a warp on: 8-warp CTAs from 96 blocks an SM (512 x 512 at level 7
+// 66 us, 4-warp CTAs 78; 1024 x 1024 at levels 6 / 8 76 / 241 us, 4-warp 88 /
+// 269; at 256 x 256, 27 an SM, 4-warp CTAs are 2-10% faster), 16-warp ones
+// from a full round of them on (2048 x 2048 at levels 6 / 8 197 / 825 us,
+// 8-warp 203 / 845; at 768 x 768 8-warp CTAs are 2-7% faster).
 static int listed_cta_warps(int64_t nblocks, int sms) {
     const int c = listed_cta_warps();
-    return c > 4 && nblocks >= (int64_t)sms * 32 * c * 2 ? c : 4;
+    if (c == 16 && nblocks >= (int64_t)sms * 32 * 16) return 16;
+    return c > 4 && nblocks >= (int64_t)sms * 96 ? 8 : 4;
 }
 
 // The batched form's per-level kernel's CTA size: the launch shape's, else 4
@@ -605,7 +609,7 @@ static cudaError_t launch_image_compacted(const GlobalTables *G, const ImageDesc
     }
     if (e == cudaSuccess) {
         // Persistent over the list, whose length only the device knows.
-        const int per_cta = cta_warps == 4 ? kWarpsPerCta * least_per_warp(L) : 32 * cta_warps;
+        const int per_cta = cta_warps == 4 ? kWarpsPerCta * least_per_warp(L) : 32;
         const int64_t most = ((int64_t)d.nblocks + per_cta - 1) / per_cta;
         const int64_t cap = (int64_t)sms * *resident;
         const int grid = (int)(most < cap ? most : cap);

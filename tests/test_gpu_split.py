@@ -51,6 +51,13 @@ def test_cta_rounds(gpu_lib, level, bh):
     check(gpu_lib, img, level, 1, None)
 
 
+@pytest.mark.parametrize("level", (4, 8, 9))
+@pytest.mark.parametrize("bw,bh", ((14591, 1), (96, 152), (305, 255), (304, 256)))
+def test_cta_sizes(gpu_lib, level, bw, bh):
+    """Either side of 96 blocks an SM (8-warp CTAs from there) and of 512 (16-warp ones)."""
+    check(gpu_lib, synth.hard_mixture_image(4 * bw, 4 * bh, seed=bw + level), level, 1, None)
+
+
 @pytest.mark.parametrize("n,decoders", ((1, (0, 1, 2, 3)), (700, (0, 1, 2, 3)), (97279, (1,)), (97281, (0,))))
 def test_refinement_counts(gpu_lib, n, decoders):
     """A warp a block below one block for each of 152 x 640 lanes, a block a lane from there on."""
