@@ -32,7 +32,8 @@ struct ImageDesc {
     float cw[3];
 };
 
-// A warp's unit of batched work: 32 consecutive blocks of one image.
+// A warp's unit of batched work: per_task (at most 32) consecutive blocks of
+// one image, the same number for every task of a batch.
 struct BatchTask {
     uint32_t image;
     uint32_t first_block;
@@ -77,11 +78,11 @@ struct BatchLists {
 // The batched form's kernel for the tasks task0 .. task0 + ntasks - 1 of a
 // byte-row batch, all of one level (each level's own code, compiled with
 // that level's plain kernels); otherwise as launch_encode_batch.
-using BatchLevelLauncher = cudaError_t (*)(const GlobalTables *, const ImageDesc *, const BatchTask *, int, int, int *,
-                                           cudaStream_t, int, const int64_t *, RefineSlot *, BatchLists);
+using BatchLevelLauncher = cudaError_t (*)(const GlobalTables *, const ImageDesc *, const BatchTask *, int, int, int,
+                                           int *, cudaStream_t, int, const int64_t *, RefineSlot *, BatchLists);
 #define ICBC_DECLARE_BATCH_LEVEL(L)                                                                                \
     cudaError_t launch_batch_level_l##L(const GlobalTables *G, const ImageDesc *images, const BatchTask *tasks,     \
-                                        int task0, int ntasks, int *counter, cudaStream_t stream, int grid,        \
+                                        int task0, int ntasks, int per_task, int *counter, cudaStream_t stream, int grid, \
                                         const int64_t *refine_base, RefineSlot *slots, BatchLists lists);
 ICBC_DECLARE_BATCH_LEVEL(0)
 ICBC_DECLARE_BATCH_LEVEL(1)
@@ -99,23 +100,23 @@ ICBC_DECLARE_BATCH_LEVEL(9)
 // weight plane), four CTAs per SM; else float rows.  With lists.list, the
 // tasks of listed images take their blocks from the lists.
 cudaError_t launch_encode_batch_float(const GlobalTables *G, const ImageDesc *images, const BatchTask *tasks,
-                                      const uint32_t *task_start, int n_images, int ntasks, int *counter,
+                                      const uint32_t *task_start, int n_images, int ntasks, int per_task, int *counter,
                                       cudaStream_t stream, int grid, const int64_t *refine_base, RefineSlot *slots,
                                       BatchLists lists);
 cudaError_t launch_encode_batch_bytes(const GlobalTables *G, const ImageDesc *images, const BatchTask *tasks,
-                                      const uint32_t *task_start, int n_images, int ntasks, int *counter,
+                                      const uint32_t *task_start, int n_images, int ntasks, int per_task, int *counter,
                                       cudaStream_t stream, int grid, const int64_t *refine_base, RefineSlot *slots,
                                       BatchLists lists);
 int batch_ctas_per_sm_float();
 int batch_ctas_per_sm_bytes();
 inline cudaError_t launch_encode_batch(const GlobalTables *G, const ImageDesc *images, const BatchTask *tasks,
-                                       const uint32_t *task_start, int n_images, int ntasks, int *counter,
+                                       const uint32_t *task_start, int n_images, int ntasks, int per_task, int *counter,
                                        cudaStream_t stream, int grid, const int64_t *refine_base = nullptr,
                                        RefineSlot *slots = nullptr, bool byte_rows = false,
                                        BatchLists lists = BatchLists{nullptr, nullptr, nullptr}) {
-    return byte_rows ? launch_encode_batch_bytes(G, images, tasks, task_start, n_images, ntasks, counter, stream, grid,
+    return byte_rows ? launch_encode_batch_bytes(G, images, tasks, task_start, n_images, ntasks, per_task, counter, stream, grid,
                                                  refine_base, slots, lists)
-                     : launch_encode_batch_float(G, images, tasks, task_start, n_images, ntasks, counter, stream, grid,
+                     : launch_encode_batch_float(G, images, tasks, task_start, n_images, ntasks, per_task, counter, stream, grid,
                                                  refine_base, slots, lists);
 }
 // First pass of a two-pass batch (byte rows): finishes the blocks of 0 or 1
@@ -123,7 +124,7 @@ inline cudaError_t launch_encode_batch(const GlobalTables *G, const ImageDesc *i
 // empty refinement slot) and lists the rest.  A grid stride over the first
 // ntasks tasks (`tasks`, or per-image offsets as for launch_encode_batch).
 cudaError_t launch_batch_trivial(const GlobalTables *G, const ImageDesc *images, const BatchTask *tasks,
-                                 const uint32_t *task_start, int n_images, int ntasks, BatchLists lists,
+                                 const uint32_t *task_start, int n_images, int ntasks, int per_task, BatchLists lists,
                                  const int64_t *refine_base, RefineSlot *slots, cudaStream_t stream, int sms);
 // Loads launch_batch_trivial's kernel (which otherwise loads on its first launch).
 void prepare_batch_trivial();
@@ -162,12 +163,16 @@ cudaError_t launch_refine_batch(const GlobalTables *G, const ImageDesc *images, 
 cudaError_t launch_simd(const GlobalTables *G, const ImageDesc *image, const BlocksSrc *blocks, const EncodeParams &p,
                         uint2 *out, float *errors, int64_t n, int level, cudaStream_t stream);
 
+// Blocks a batched task takes, for `blocks` in all: 32, or as few as give
+// every resident warp one.
+int batch_task_blocks(int64_t blocks);
+
 // Launch shape of the plain kernels of a level (autotuned or default).
 struct LaunchShape {
     int groups_per_warp;
     bool persistent;
     int cta_warps;        // the listed pass's CTA size (0: the level's default)
-    int batch_cta_warps;  // the batched form's per-level kernel's (0: 4)
+    int batch_cta_warps;  // the batched form's per-level kernel's (0: the default)
 };
 LaunchShape launch_shape(int level);
 

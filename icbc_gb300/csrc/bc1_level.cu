@@ -349,7 +349,7 @@ __global__ void __launch_bounds__(NW * 32, 512 / (NW * 32))
 template <int LV, int NW>
 __global__ void __launch_bounds__(NW * 32, 512 / (NW * 32))
     k_batch_level_cta(const GlobalTables *G, const ImageDesc *images, const BatchTask *tasks, int task0, int ntasks,
-                      int *counter, const int64_t *refine_base, RefineSlot *slots, BatchLists lists) {
+                      int per_task, int *counter, const int64_t *refine_base, RefineSlot *slots, BatchLists lists) {
     extern __shared__ __align__(16) unsigned char smem[];
     SharedTables &T = *reinterpret_cast<SharedTables *>(smem);
     stage_tables(T, G);
@@ -372,10 +372,10 @@ __global__ void __launch_bounds__(NW * 32, 512 / (NW * 32))
         const ImageDesc &d = images[task.image];
         const int64_t lb = lists.list ? lists.list_base[task.image] : -1;
         int64_t b = (int64_t)task.first_block + lane;
-        bool active = has_task && b < d.nblocks;
+        bool active = has_task && lane < per_task && b < d.nblocks;
         if (has_task && lb >= 0) {
             const int64_t n = lists.listed[task.image];
-            active = b < n;  // tasks past the list's end: finished by the first pass
+            active = lane < per_task && b < n;  // tasks past the list's end: finished by the first pass
             b = active ? (int64_t)lists.list[lb + b] : 0;
         }
         if (lane == 0)
@@ -429,9 +429,9 @@ __global__ void __launch_bounds__(NW * 32, 512 / (NW * 32))
 template <int LV>
 __global__ void __launch_bounds__(kWarpsPerCta * 32, 4)
     k_batch_level(const GlobalTables *G, const ImageDesc *images, const BatchTask *tasks, int task0, int ntasks,
-                  int *counter, const int64_t *refine_base, RefineSlot *slots, BatchLists lists) {
+                  int per_task, int *counter, const int64_t *refine_base, RefineSlot *slots, BatchLists lists) {
     extern __shared__ __align__(16) unsigned char smem[];
-    run_batch<true, LV>(G, smem, images, tasks, nullptr, 0, task0, ntasks, counter, refine_base, slots, lists);
+    run_batch<true, LV>(G, smem, images, tasks, nullptr, 0, task0, ntasks, per_task, counter, refine_base, slots, lists);
 }
 
 constexpr int L = ICBC_LEVEL;
@@ -550,12 +550,14 @@ static int listed_cta_warps(int64_t nblocks, int sms) {
     return c > 4 && nblocks >= (int64_t)sms * 96 ? 8 : 4;
 }
 
-// The batched form's per-level kernel's CTA size: the launch shape's, else 4
-// (on a mixed batch of small images CTA-wide searches do not pay: a round's
-// tasks often differ in decoder or colour weights).
+// The batched form's per-level kernel's CTA size: the launch shape's, else 8
+// from level 4 on, where the CTA's stages in step keep the long per-block code
+// in the instruction cache (300 images of 64 to 2048 a side, all levels: 7.21
+// ms with 4-warp CTAs, 6.23 with 8, 6.43 with 16; 400 of the mixed batch 6.53
+// / 6.34 / 6.45; below level 4 either size takes the same time).
 static int batch_cta_warps() {
     const int c = launch_shape(L).batch_cta_warps;
-    return c == 8 || c == 16 ? c : 4;
+    return c == 4 || c == 8 || c == 16 ? c : L >= 4 ? 8 : 4;
 }
 
 // Shared-memory limit of a listed-pass kernel and, once, its resident CTAs per SM.
@@ -659,8 +661,8 @@ cudaError_t ICBC_CAT(launch_blocks_l, ICBC_LEVEL)(const GlobalTables *G, const B
 }
 
 cudaError_t ICBC_CAT(launch_batch_level_l, ICBC_LEVEL)(const GlobalTables *G, const ImageDesc *images,
-                                                        const BatchTask *tasks, int task0, int ntasks, int *counter,
-                                                        cudaStream_t stream, int grid, const int64_t *refine_base,
+                                                        const BatchTask *tasks, int task0, int ntasks, int per_task,
+                                                        int *counter, cudaStream_t stream, int grid, const int64_t *refine_base,
                                                         RefineSlot *slots, BatchLists lists) {
     // `grid` counts 4-warp CTAs; a CTA-wide kernel gets as many warps in all.
     const int cta_warps = Level<L>::cluster && (L < 9 || refine_base) ? batch_cta_warps() : 4;
@@ -673,17 +675,17 @@ cudaError_t ICBC_CAT(launch_batch_level_l, ICBC_LEVEL)(const GlobalTables *G, co
         const int want = (grid * kWarpsPerCta + cta_warps - 1) / cta_warps;
         const int ctas = std::max(1, std::min(want, current_sm_count() * *resident));
         if (cta_warps == 16)
-            k_batch_level_cta<L, 16><<<ctas, 16 * 32, smem, stream>>>(G, images, tasks, task0, ntasks, counter,
+            k_batch_level_cta<L, 16><<<ctas, 16 * 32, smem, stream>>>(G, images, tasks, task0, ntasks, per_task, counter,
                                                                        refine_base, slots, lists);
         else
-            k_batch_level_cta<L, 8><<<ctas, 8 * 32, smem, stream>>>(G, images, tasks, task0, ntasks, counter,
+            k_batch_level_cta<L, 8><<<ctas, 8 * 32, smem, stream>>>(G, images, tasks, task0, ntasks, per_task, counter,
                                                                      refine_base, slots, lists);
         return cudaGetLastError();
     }
     const size_t smem = smem_bytes_byte_rows();
     cudaError_t e = cudaFuncSetAttribute(k_batch_level<L>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    k_batch_level<L><<<grid, kWarpsPerCta * 32, smem, stream>>>(G, images, tasks, task0, ntasks, counter, refine_base,
+    k_batch_level<L><<<grid, kWarpsPerCta * 32, smem, stream>>>(G, images, tasks, task0, ntasks, per_task, counter, refine_base,
                                                                slots, lists);
     return cudaGetLastError();
 }

@@ -294,6 +294,15 @@ int ensure_tables_on_device(const GlobalTables **out) { return ensure_device_tab
 
 int current_sm_count() { return sm_count(); }
 
+// A small batch in tasks of 32 blocks would leave most warps without one, and
+// a warp's time grows with its blocks: it takes tasks of as few blocks as give
+// each of the resident warps (16 an SM) one (10 images of up to 256 x 256:
+// 169 -> 84 us with the 8-warp CTAs; 30 of up to 512 x 512: 410 -> 371).
+int batch_task_blocks(int64_t blocks) {
+    const int64_t warps = 16 * (int64_t)sm_count();
+    return (int)std::max<int64_t>(1, std::min<int64_t>(32, (blocks + warps - 1) / warps));
+}
+
 }  // namespace icbc_gpu
 
 // Relative cost of a 32-block task per level, used to order batched work
@@ -512,7 +521,7 @@ int icbc_gpu_batch_create(const icbc_gpu_image *images, int n_images, icbc_gpu_b
     const GlobalTables *G = nullptr;
     int st = ensure_device_tables(&G);
     if (st) return st;
-    // Tasks of 32 blocks, most expensive level first; inside a level the
+    // Tasks of up to 32 blocks, most expensive level first; inside a level the
     // images with the same decoder and colour weights together (the CTA-wide
     // kernels search a round's blocks together only when its tasks share
     // them), larger images first, so the tail of each launch is cheap work.
@@ -537,12 +546,16 @@ int icbc_gpu_batch_create(const icbc_gpu_image *images, int n_images, icbc_gpu_b
     });
     std::vector<int> own;  // images that get their level's own launch
     std::vector<BatchTask> tasks;
+    int64_t shared_blocks = 0;
+    for (int i : order)
+        if (descs[i].nblocks < kOwnLaunchBlocks) shared_blocks += descs[i].nblocks;
+    const int per_task = batch_task_blocks(shared_blocks);
     for (int i : order) {
         if (descs[i].nblocks >= kOwnLaunchBlocks) {
             own.push_back(i);
             continue;
         }
-        for (int64_t b = 0; b < descs[i].nblocks; b += 32) tasks.push_back(BatchTask{(uint32_t)i, (uint32_t)b});
+        for (int64_t b = 0; b < descs[i].nblocks; b += per_task) tasks.push_back(BatchTask{(uint32_t)i, (uint32_t)b});
     }
     if (tasks.size() > 0x7fffffff) return ICBC_GPU_ERR_INVALID_ARGUMENT;
     // Refinement slots of the level-9 images, in task order; then those of
@@ -658,7 +671,7 @@ int icbc_gpu_batch_create(const icbc_gpu_image *images, int n_images, icbc_gpu_b
         if (e1 == cudaSuccess && B->d_list) {
             e1 = cudaMemsetAsync(B->d_listed, 0, sizeof(unsigned int) * n_images, cs);
             if (e1 == cudaSuccess)
-                e1 = launch_batch_trivial(G, B->d_images, B->d_tasks, nullptr, n_images, B->ntasks_listed, lists,
+                e1 = launch_batch_trivial(G, B->d_images, B->d_tasks, nullptr, n_images, B->ntasks_listed, per_task, lists,
                                           B->d_refine_base, B->d_slots, cs, sm_count());
         }
         cudaError_t e2 = e1;
@@ -670,13 +683,13 @@ int icbc_gpu_batch_create(const icbc_gpu_image *images, int n_images, icbc_gpu_b
                 const int grid = std::min(B->grid, (n + kWarpsPerCta - 1) / kWarpsPerCta);  // a task per warp at most
                 e2 = cudaStreamWaitEvent(lv_stream[l], fork, 0);
                 if (e2 == cudaSuccess)
-                    e2 = kBatchLevelLaunch[l](G, B->d_images, B->d_tasks, lv_begin[l], n, B->d_counter + 1 + l,
+                    e2 = kBatchLevelLaunch[l](G, B->d_images, B->d_tasks, lv_begin[l], n, per_task, B->d_counter + 1 + l,
                                               lv_stream[l], grid, B->d_refine_base, B->d_slots, lists);
                 if (e2 == cudaSuccess) e2 = cudaEventRecord(lv_done[l], lv_stream[l]);
                 if (e2 == cudaSuccess) e2 = cudaStreamWaitEvent(cs, lv_done[l], 0);
             }
         } else if (e2 == cudaSuccess && B->ntasks) {
-            e2 = launch_encode_batch(G, B->d_images, B->d_tasks, nullptr, n_images, B->ntasks, B->d_counter, cs,
+            e2 = launch_encode_batch(G, B->d_images, B->d_tasks, nullptr, n_images, B->ntasks, per_task, B->d_counter, cs,
                                      B->grid, B->d_refine_base, B->d_slots, byte_rows, lists);
         }
         if (e2 == cudaSuccess && refine_total) {

@@ -355,16 +355,17 @@ int icbc_gpu_compress_bc1_mips(const icbc_gpu_image *image, int32_t levels, void
  * each warp searching its own 32 blocks' cluster combinations; 8 or 16 =
  * CTAs of that many warps moving through the encoder's stages together, the
  * combinations of all the CTA's blocks searched by all its threads (an image
- * too small for two rounds of such CTAs on every SM takes 4); 0 = the
- * level's default.  Defaults: 1 / persistent at levels 0-1, 2 / not
- * persistent at levels 2-9, cta_warps 16 from level 4 on (else 4),
- * batch_cta_warps 4.  Not for use while launches run or batches are
- * created. */
+ * of fewer than 512 blocks an SM takes 8 instead of 16, one of fewer than 96
+ * takes 4); 0 = the level's default.  An image too small to give every
+ * resident warp 32 blocks takes smaller shares whatever the shape.  Defaults:
+ * 1 / persistent at levels 0-1, 2 / not persistent at levels 2-9, cta_warps
+ * 16 and batch_cta_warps 8 from level 4 on (else 4).  Not for use while
+ * launches run or batches are created. */
 typedef struct icbc_gpu_launch_config {
     int32_t groups_per_warp;
     int32_t persistent;
     int32_t cta_warps;
-    int32_t batch_cta_warps;  /* 0 = 4 */
+    int32_t batch_cta_warps;  /* 0 = the default: 8 from level 4 on, else 4 */
 } icbc_gpu_launch_config;
 int icbc_gpu_set_launch_config(int level, const icbc_gpu_launch_config *config);
 int icbc_gpu_get_launch_config(int level, icbc_gpu_launch_config *config);

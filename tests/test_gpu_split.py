@@ -67,3 +67,30 @@ def test_refinement_counts(gpu_lib, n, decoders):
             b, e = gpu_lib.compress_blocks(cols, w, 9, dec, (0.299, 0.587, 0.114), tc, tcb)
             ob, oe = O.compress_blocks(cols, w, 9, dec, (0.299, 0.587, 0.114), tc, tcb, nthreads=16)
             assert np.array_equal(b, ob) and np.array_equal(e.view(np.uint32), oe.view(np.uint32))
+
+
+@pytest.mark.parametrize("sides", ((4, 9, 1), (40, 64, 33, 8), (300, 500, 260, 410, 77)))
+def test_small_batches(gpu_lib, sides):
+    """Batches below 32 blocks for every warp take smaller tasks: some past a list's end, ragged images, mixed
+    levels, decoders and colour weights in one CTA's round."""
+    import torch
+    ig = gpu_lib
+    keep, descs, cases = [], [], []
+    for k, side in enumerate(sides):
+        for level in range(10):
+            img = synth.quality_sweep_image(side + level, side, seed=k) if side >= 33 else synth.hard_mixture_image(
+                side + level, side, seed=k)
+            t, n = torch.from_numpy(img).cuda(), ig.blocks_of(side + level, side)
+            out, err = torch.zeros((n, 8), dtype=torch.uint8, device="cuda"), torch.zeros(n, device="cuda")
+            cw = (1.0, 1.0, 1.0) if level % 2 else (0.299, 0.587, 0.114)
+            keep += [t, out, err]
+            descs.append(ig.image_desc(t, level, out, err, (k + level) % 4, cw, level % 2))
+            cases.append((img, level, (k + level) % 4, cw, level % 2, out, err))
+    b = ig.Batch(descs, keepalive=keep)
+    b.launch()
+    torch.cuda.synchronize()
+    for img, level, dec, cw, mode, out, err in cases:
+        ob, oe = O.encode_image(img, level, dec, cw, mode, None, True, True, nthreads=16)
+        assert np.array_equal(out.cpu().numpy(), ob), (img.shape, level)
+        assert np.array_equal(err.cpu().numpy().view(np.uint32), oe.view(np.uint32))
+    b.close()
