@@ -29,7 +29,9 @@ __device__ __forceinline__ BatchTask batch_task(const BatchTask *tasks, const ui
 template <bool BYTES, int L, bool DEFER>
 __device__ __forceinline__ float encode_task(const WarpCtx &w, const ImageDesc &d, const EncodeParams &p, bool active,
                                              uint32_t &c0, uint32_t &c1, uint32_t &idx, bool &pending) {
-    if constexpr (BYTES)
+    if constexpr (BYTES && L < 2)
+        return encode_warp_ex<L, DEFER>(w, image_row(w), p, active, c0, c1, idx, pending);
+    else if constexpr (BYTES)
         return encode_warp_ex<L, DEFER>(w, byte_row(w, d.weight_mode == ICBC_GPU_WEIGHTS_ALPHA), p, active, c0, c1,
                                         idx, pending);
     else
@@ -107,7 +109,8 @@ __device__ __forceinline__ void run_batch(const GlobalTables *G, unsigned char *
         const WarpCtx w = BYTES ? warp_ctx_byte_rows(smem, T, G, p.decoder) : warp_ctx<9>(smem, T, G, p.decoder);
         __syncwarp();
         if (active) {
-            if (BYTES) load_image_block_bytes(d, b, reinterpret_cast<uint32_t *>(w.in) + lane * kInWordsByte);
+            if (BYTES && level < 2) load_image_row(d, b, w.sat + lane * kSatStride, T.lut255);
+            else if (BYTES) load_image_block_bytes(d, b, reinterpret_cast<uint32_t *>(w.in) + lane * kInWordsByte);
             else load_image_block(d, b, w.in + lane * kInStride, T.lut255);
         }
         __syncwarp();

@@ -47,6 +47,13 @@ constexpr int kInWordsByte = 17;
 constexpr size_t kWarpFloatsByte = 32 * kInWordsByte + 32 * kSatStride + 64 + 32;
 __host__ __device__ constexpr size_t smem_bytes_byte_rows() { return sizeof(SharedTables) + kWarpsPerCta * 4 * kWarpFloatsByte; }
 
+// Levels 0-1 of the RGBA8 image kernels: the colour tables, and per warp 32
+// float4 texel rows of kSatStride floats and 32 palettes (ImageRow), 44 KB a
+// CTA: five CTAs per SM.  In a byte-row layout, whose SAT rows these levels
+// do not use, the texels lie in `sat` and the palettes in `in`.
+constexpr size_t kWarpFloatsImage = 32 * kSatStride + 4 * 32 * 4;
+__host__ __device__ constexpr size_t smem_bytes_image() { return kColorTableBytes + kWarpsPerCta * 4 * kWarpFloatsImage; }
+
 // Options of each quality level (setup_options, icbc.h:3663-3731).
 template <int L>
 struct Level {
@@ -297,7 +304,7 @@ template <class Row>
 __device__ __forceinline__ bool optimize_end_points4(const Row &row, uint32_t indices, V3 &a, V3 &b) {
     float alpha2 = 0.0f, beta2 = 0.0f, ab = 0.0f;
     V3 ax = v3(0.0f, 0.0f, 0.0f), bx = v3(0.0f, 0.0f, 0.0f);
-#pragma unroll 1
+#pragma unroll Row::kUnroll
     for (int i = 0; i < 16; i++) {
         const uint32_t bits = indices >> (2 * i);
         // beta = bits & 1, and for bits & 2 (1 + beta) / 3: the two possible
@@ -323,6 +330,8 @@ __device__ __forceinline__ bool optimize_end_points4(const Row &row, uint32_t in
 // Box fit: fit_colors_bbox, inset_bbox, select_diagonal (icbc.h:3313-3368).
 // `colors`: the reduced colours in a SAT row (SatColors) or a texel row.
 struct SatColors {
+    static constexpr bool kBounded = false;
+    static constexpr int kUnroll = 1;
     const float *p;
     __device__ __forceinline__ V3 color(int i) const { return xyz(ld4(p + 4 * i)); }
 };
@@ -331,10 +340,16 @@ template <class C>
 __device__ __forceinline__ void box_fit(const C &colors, int count, V3 &c0, V3 &c1) {
     c0 = v3(0.0f, 0.0f, 0.0f);
     c1 = v3(1.0f, 1.0f, 1.0f);
+#pragma unroll C::kUnroll
     for (int i = 0; i < count; i++) {
         const V3 c = colors.color(i);
-        c0 = vmax(c0, c);
-        c1 = vmin(c1, c);
+        if (C::kBounded) {  // no NaN and no -0: the reference's max and min are fmaxf and fminf
+            c0 = v3(fmaxf(c0.x, c.x), fmaxf(c0.y, c.y), fmaxf(c0.z, c.z));
+            c1 = v3(fminf(c1.x, c.x), fminf(c1.y, c.y), fminf(c1.z, c.z));
+        } else {
+            c0 = vmax(c0, c);
+            c1 = vmin(c1, c);
+        }
     }
     const float bias = (8.0f / 255.0f) / 16.0f;
     const V3 d = c0 - c1;
@@ -343,6 +358,7 @@ __device__ __forceinline__ void box_fit(const C &colors, int count, V3 &c0, V3 &
     c1 = saturate(c1 + inset);
     const V3 center = (c0 + c1) * 0.5f;
     float cov_xz = 0.0f, cov_yz = 0.0f;
+#pragma unroll C::kUnroll
     for (int i = 0; i < count; i++) {
         const V3 t = colors.color(i) - center;
         cov_xz += t.x * t.z;

@@ -74,20 +74,34 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32) k_encode_blocks(const Globa
     }
 }
 
+// Levels 0-1 take ImageRows: one 16-byte load a texel and pass instead of four
+// loads, the chosen palette entry by a load instead of a 4-way select, four
+// texels at a time in flight (2: 2% slower, 8: 12%, 16: 70%, instruction
+// fetch).  Bound by issue (3,580 instructions a warp, 4,330 before): 4096 x
+// 4096 at level 1 134 us, before 161; at level 0 80, before 93.
 template <int L, bool DEFER>
 __global__ void __launch_bounds__(kWarpsPerCta * 32) k_encode_image(const GlobalTables *G, ImageDesc d, EncodeParams p,
                                                                     int per_warp, RefineSlot *st) {
     extern __shared__ __align__(16) unsigned char smem[];
     SharedTables &T = *reinterpret_cast<SharedTables *>(smem);
-    stage_tables(T, G);
-    const WarpCtx w = warp_ctx<L>(smem, T, G, p.decoder);
+    WarpCtx w;
+    if constexpr (L < 2) {
+        stage_color_tables(T, G);
+        w = warp_ctx_image(smem, T, G, p.decoder);
+    } else {
+        stage_tables(T, G);
+        w = warp_ctx<L>(smem, T, G, p.decoder);
+    }
     const int64_t groups = (d.nblocks + per_warp - 1) / per_warp;
     for (int64_t g = (int64_t)blockIdx.x * kWarpsPerCta + (threadIdx.x >> 5); g < groups;
          g += (int64_t)gridDim.x * kWarpsPerCta) {
         const int64_t b = g * per_warp + w.lane;
         const bool active = w.lane < per_warp && b < d.nblocks;
         __syncwarp();
-        if (active) load_image_block(d, b, w.in + w.lane * kInStride, T.lut255);
+        if (active) {
+            if constexpr (L < 2) load_image_row(d, b, w.sat + w.lane * kSatStride, T.lut255);
+            else load_image_block(d, b, w.in + w.lane * kInStride, T.lut255);
+        }
         __syncwarp();
         uint32_t c0 = 0, c1 = 0, idx = 0;
         if (L >= 4 && active) {
@@ -97,7 +111,9 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32) k_encode_image(const Global
             idx = prev.y;
         }
         bool pending;
-        const float e = encode_warp_ex<L, DEFER>(w, float_row(w), p, active, c0, c1, idx, pending);
+        float e;
+        if constexpr (L < 2) e = encode_warp_ex<L, DEFER>(w, image_row(w), p, active, c0, c1, idx, pending);
+        else e = encode_warp_ex<L, DEFER>(w, float_row(w), p, active, c0, c1, idx, pending);
         if (active) {
             d.out[b] = make_uint2(c0 | (c1 << 16), idx);
             if (d.errors) d.errors[b] = e;
@@ -643,7 +659,7 @@ static cudaError_t launch_image(const GlobalTables *G, const ImageDesc &d, const
                        },
                        G, &d, nullptr, p, d.out, d.errors, ext_st, ext_counter);
     }
-    return run(k_encode_image<L, kDefer>, smem_bytes(Level<L>::cluster), g_resident_image, d.nblocks, sms, stream,
+    return run(k_encode_image<L, kDefer>, L < 2 ? smem_bytes_image() : smem_bytes(Level<L>::cluster), g_resident_image, d.nblocks, sms, stream,
                [&](int grid, size_t smem, int per_warp, RefineSlot *slots) {
                    k_encode_image<L, kDefer><<<grid, kWarpsPerCta * 32, smem, stream>>>(G, d, p, per_warp, slots);
                },

@@ -94,6 +94,24 @@ __device__ __forceinline__ void load_image_block(const ImageDesc &d, int64_t b, 
     }
 }
 
+// The same into an ImageRow's 16-byte aligned row, a texel a store.
+__device__ __forceinline__ void load_image_row(const ImageDesc &d, int64_t b, float *row, const float *lut) {
+    const int bx = (int)(b % d.bw), by = (int)(b / d.bw);
+    uint32_t px[16];
+    fetch_image_block(d, b, px);
+#pragma unroll
+    for (int t = 0; t < 16; t++) {
+        float w = 1.0f;
+        if (d.weight_mode == 1) {
+            w = lut[px[t] >> 24];
+        } else if (d.weight_mode == 2) {
+            const int x = min(4 * bx + (t & 3), d.width - 1), y = min(4 * by + (t >> 2), d.height - 1);
+            w = __ldg(d.weight_plane + (int64_t)y * d.weight_pitch + x);
+        }
+        st4(row + 4 * t, make_float4(lut[px[t] & 255], lut[(px[t] >> 8) & 255], lut[(px[t] >> 16) & 255], w));
+    }
+}
+
 // One block of an RGBA8 image into this lane's byte row (the words as they are).
 __device__ __forceinline__ void load_image_block_bytes(const ImageDesc &d, int64_t b, uint32_t *row) {
     uint32_t px[16];
@@ -106,6 +124,14 @@ __device__ __forceinline__ void stage_tables(SharedTables &T, const GlobalTables
     const uint4 *src = reinterpret_cast<const uint4 *>(&G->s);
     uint4 *dst = reinterpret_cast<uint4 *>(&T);
     for (int i = threadIdx.x; i < (int)(sizeof(SharedTables) / 16); i += blockDim.x) dst[i] = src[i];
+    __syncthreads();
+}
+
+// The tables that levels 0-1 use.
+__device__ __forceinline__ void stage_color_tables(SharedTables &T, const GlobalTables *G) {
+    const uint4 *src = reinterpret_cast<const uint4 *>(&G->s);
+    uint4 *dst = reinterpret_cast<uint4 *>(&T);
+    for (int i = threadIdx.x; i < (int)(kColorTableBytes / 16); i += blockDim.x) dst[i] = src[i];
     __syncthreads();
 }
 
@@ -140,6 +166,22 @@ __device__ __forceinline__ WarpCtx warp_ctx_byte_rows(unsigned char *smem, const
     w.info = reinterpret_cast<int *>(base + 32 * kInWordsByte + 32 * kSatStride + 64);
     w.lane = threadIdx.x & 31;
     return w;
+}
+
+// The warp's context at levels 0-1 (ImageRow): texels in `sat`, palettes in `in`.
+__device__ __forceinline__ WarpCtx warp_ctx_image(unsigned char *smem, const SharedTables &T, const GlobalTables *G,
+                                                  int decoder) {
+    WarpCtx w{};
+    w.T = &T;
+    w.D = &G->dec[decoder];
+    w.sat = reinterpret_cast<float *>(smem + kColorTableBytes) + (threadIdx.x >> 5) * kWarpFloatsImage;
+    w.in = w.sat + 32 * kSatStride;
+    w.lane = threadIdx.x & 31;
+    return w;
+}
+
+__device__ __forceinline__ ImageRow image_row(const WarpCtx &w) {
+    return ImageRow{w.sat + w.lane * kSatStride, reinterpret_cast<float4 *>(w.in) + w.lane};
 }
 
 __device__ __forceinline__ ByteRow byte_row(const WarpCtx &w, int alpha) {
