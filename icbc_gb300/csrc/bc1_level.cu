@@ -644,10 +644,21 @@ static cudaError_t launch_image_compacted(const GlobalTables *G, const ImageDesc
     return e != cudaSuccess ? e : f;
 }
 
+// Whether an image of `nblocks` blocks is encoded in one pass.  Two passes
+// keep blocks of 0 or 1 colours out of the searching warps, but cost a
+// scratch allocation, a memset and a second kernel that waits for the first.
+// One pass up to 512 blocks an SM (a block for every lane that fits), from
+// level 7 on, where a warp's search outweighs that, up to 96 (where the
+// CTA-wide pass begins).  One / two passes, us, no allocations by the caller:
+// level 4 at 64 x 64 17 / 32, 512 x 512 29 / 43, 1024 x 1024 37 / 49, 1448 x
+// 1448 64 / 59; level 6 27 / 41, 47 / 55, 65 / 69, 123 / 120; level 8 30 /
+// 43, 115 / 105 (at 384 x 384 84 / 88).
+static bool one_pass(int64_t nblocks, int sms) { return nblocks < (int64_t)sms * (L >= 7 ? 96 : 512); }
+
 static cudaError_t launch_image(const GlobalTables *G, const ImageDesc &d, const EncodeParams &p, cudaStream_t stream,
                                 int sms, RefineSlot *ext_st, unsigned long long *ext_counter) {
     if constexpr (kCompact) {
-        if (use_byte_rows(d) && d.nblocks < (int64_t(1) << 32))
+        if (use_byte_rows(d) && d.nblocks < (int64_t(1) << 32) && !one_pass(d.nblocks, sms))
             return launch_image_compacted(G, d, p, stream, sms, ext_st, ext_counter);
     }
     if constexpr (Level<L>::cluster) {
