@@ -454,72 +454,6 @@ __device__ __forceinline__ float refine(const WarpCtx &w, const Row &row, const 
     return best;
 }
 
-// One block's refinement state, for refinement run one step at a time.
-struct RefineLane {
-    uint32_t c0, c1, idx, base_idx;
-    float best;
-    int i, last;
-};
-
-// `lut`: the exact table of i / 255.0f.
-template <class Row>
-__device__ __forceinline__ void refine_begin(const WarpCtx &w, const float *lut, const Row &row, const EncodeParams &p,
-                                             float error, uint32_t c0, uint32_t c1, uint32_t idx, RefineLane &s) {
-    s.c0 = c0;
-    s.c1 = c1;
-    s.idx = idx;
-    s.best = error;
-    s.i = 0;
-    s.last = 0;
-    s.base_idx = indices_generic<4>(row, p.cw, palette_f(c0, c1, p.decoder, lut, w.D));
-}
-
-// block_error with the palette in shared memory: entry e of this lane at
-// pal[32 * e] (a warp's palettes laid out entry-major, so the 16-byte loads of
-// any 8 lanes fall in 8 bank groups whatever their indices).  One load per
-// texel instead of a 4-way select; the same floats in the same order.
-template <int UNROLL = 1, class Row>
-__device__ __forceinline__ float block_error_pal(const Row &row, V3 cw, const PalF &p, float4 *pal,
-                                                 uint32_t indices) {
-#pragma unroll
-    for (int e = 0; e < 4; e++) pal[32 * e] = make_float4(p.c[e].x, p.c[e].y, p.c[e].z, 0.0f);
-    float error = 0.0f;
-#pragma unroll UNROLL
-    for (int t = 0; t < 16; t++) {
-        const float4 q = pal[32 * ((indices >> (2 * t)) & 3)];
-        error += row.weight(t) * texel_mse(v3(q.x, q.y, q.z), row.color(t), cw);
-    }
-    return error;
-}
-
-// Iteration s.i of refine_endpoints (icbc.h:3614-3648), one trip of
-// refine()'s loop but for its index update: when the step is accepted it
-// takes the candidate and returns true with the candidate's palette in `pr`,
-// and s.base_idx must be set to indices_generic(row, cw, pr) before the next
-// iteration (the caller computes it, across lanes).  `stop`: the loop would
-// stop after this iteration.  With `pal` (this lane's shared-memory palette
-// slot, block_error_pal) the step's error picks entries by a load.
-template <class Row>
-__device__ __forceinline__ bool refine_try(const WarpCtx &w, const float *lut, const Row &row, const EncodeParams &p,
-                                           RefineLane &s, PalF &pr, bool &stop, float4 *pal = nullptr) {
-    const int8_t *d = c_deltas[s.i & 15];
-    uint32_t r0 = s.c0, r1 = s.c1;
-    refine_candidate(s.i, d[0], d[1], d[2], p, r0, r1);
-    pr = palette_f(r0, r1, p.decoder, lut, w.D);
-    const float e = pal ? block_error_pal<4>(row, p.cw, pr, pal, s.base_idx) : block_error<4>(row, p.cw, pr, s.base_idx);
-    const bool accept = e < s.best;
-    if (accept) {
-        s.best = e;
-        s.c0 = r0;
-        s.c1 = r1;
-        s.idx = s.base_idx;
-        s.last = s.i;
-    }
-    s.i++;
-    stop = (s.i - 1 - s.last > 32) || s.i == 256;
-    return accept;
-}
-
 // Per-block hand-over from the encode kernel to the refinement kernel.
 struct RefineSlot {
     float error;       // compress_bc1's error before refinement

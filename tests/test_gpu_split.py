@@ -58,9 +58,10 @@ def test_cta_sizes(gpu_lib, level, bw, bh):
     check(gpu_lib, synth.hard_mixture_image(4 * bw, 4 * bh, seed=bw + level), level, 1, None)
 
 
-@pytest.mark.parametrize("n,decoders", ((1, (0, 1, 2, 3)), (700, (0, 1, 2, 3)), (97279, (1,)), (97281, (0,))))
+@pytest.mark.parametrize("n,decoders", ((1, (0, 1, 2, 3)), (700, (0, 1, 2, 3)), (8191, (1,)), (8193, (2,)),
+                                        (98303, (1,)), (98305, (0,))))
 def test_refinement_counts(gpu_lib, n, decoders):
-    """A warp a block below one block for each of 152 x 640 lanes, a block a lane from there on."""
+    """32 lanes a block below 8,192 blocks, 8 below 98,304, 4 from there on."""
     cols, w = synth.mixed_blocks(n, seed=n)
     for dec in decoders:
         for tc, tcb in ((True, True), (False, False)):
