@@ -317,7 +317,7 @@ template <int L, bool DEFER, int NW>
 __global__ void __launch_bounds__(NW * 32, 512 / (NW * 32))
     k_image_listed_cta(const GlobalTables *G, ImageDesc d, EncodeParams p, const uint32_t *list,
                        const unsigned int *listed, RefineSlot *st) {
-    const int64_t n = *listed;
+    const int64_t n = list ? (int64_t)*listed : d.nblocks;  // no list: every block of the image
     const int per_cta = balanced_share(n, gridDim.x, 32 * NW, 1);
     const int64_t groups = (n + per_cta - 1) / per_cta;
     if ((int64_t)blockIdx.x >= groups) return;  // the whole CTA has no work
@@ -332,7 +332,7 @@ __global__ void __launch_bounds__(NW * 32, 512 / (NW * 32))
     for (int64_t grp = blockIdx.x; grp < groups; grp += gridDim.x) {
         const int64_t k = grp * per_cta + threadIdx.x;
         const bool active = (int)threadIdx.x < per_cta && k < n;
-        const int64_t b = active ? (int64_t)list[k] : 0;
+        const int64_t b = !active ? 0 : list ? (int64_t)list[k] : k;
         __syncwarp();
         if (active) load_image_block_bytes(d, b, in + threadIdx.x * kInWordsByte);
         __syncwarp();
@@ -576,6 +576,18 @@ static int batch_cta_warps() {
     return c == 4 || c == 8 || c == 16 ? c : L >= 4 ? 8 : 4;
 }
 
+// Whether the CTA-wide pass takes all of an image's blocks instead of a list,
+// at levels 4-7: up to 512 blocks an SM, 900 at levels 6-7, where the first
+// pass costs more (its allocation, memset and wait included) than it keeps out
+// of the CTA's stages.  With / without, us: level 5 at 512 x 512 37 / 51, 1100
+// x 1100 45 / 57, 1448 x 1448 82 / 70; level 7 49 / 62, 81 / 92, 140 / 154,
+// 2048 x 2048 283 / 271.  At levels 8-9, where a CTA's blocks of 0 or 1
+// colours unbalance the searches, the list stays (level 8 at 1100 x 1100 274 /
+// 252).
+static bool one_cta_pass(int64_t nblocks, int sms) {
+    return L >= 4 && L <= 7 && nblocks < (int64_t)sms * (L >= 6 ? 900 : 512);
+}
+
 // Shared-memory limit of a listed-pass kernel and, once, its resident CTAs per SM.
 template <class K>
 static cudaError_t listed_attributes(K kernel, int warps, size_t smem, int *resident) {
@@ -588,7 +600,8 @@ static cudaError_t listed_attributes(K kernel, int warps, size_t smem, int *resi
     return e;
 }
 
-// The two passes of kCompact levels, with the list (and at level 9 the
+// The passes of kCompact levels -- the CTA-wide one alone for smaller images
+// (one_cta_pass) -- with the list (and at level 9 the
 // refinement hand-over, unless the caller gives one) in stream-ordered
 // scratch; level 9 then runs its refinement pass over every block.
 static cudaError_t launch_image_compacted(const GlobalTables *G, const ImageDesc &d, const EncodeParams &p,
@@ -604,23 +617,24 @@ static cudaError_t launch_image_compacted(const GlobalTables *G, const ImageDesc
     else if (cta_warps == 8) e = listed_attributes(k_image_listed_cta<L, kDefer, 8>, 8, smem, resident);
     else e = listed_attributes(k_image_listed<L, kDefer>, kWarpsPerCta, smem, resident);
     if (e != cudaSuccess) return e;
-    const size_t list_bytes = ((size_t)d.nblocks * 4 + 15) / 16 * 16;
+    const bool listing = cta_warps == 4 || !one_cta_pass(d.nblocks, sms);
+    const size_t list_bytes = listing ? ((size_t)d.nblocks * 4 + 15) / 16 * 16 + 16 : 0;
     const size_t slot_bytes = (kDefer && !ext_st) ? ((size_t)d.nblocks * sizeof(RefineSlot) + 15) / 16 * 16 + 16 : 0;
     void *scratch = nullptr;
-    e = scratch_alloc(&scratch, list_bytes + 16 + slot_bytes, stream);
+    if (list_bytes + slot_bytes) e = scratch_alloc(&scratch, list_bytes + slot_bytes, stream);
     if (e != cudaSuccess) return e;
     char *base = static_cast<char *>(scratch);
-    uint32_t *list = reinterpret_cast<uint32_t *>(base);
-    unsigned int *listed = reinterpret_cast<unsigned int *>(base + list_bytes);
+    uint32_t *list = listing ? reinterpret_cast<uint32_t *>(base) : nullptr;
+    unsigned int *listed = listing ? reinterpret_cast<unsigned int *>(base + list_bytes - 16) : nullptr;
     RefineSlot *st = ext_st;
     unsigned long long *counter = ext_counter;
     if (kDefer && !ext_st) {
-        st = reinterpret_cast<RefineSlot *>(base + list_bytes + 16);
-        counter = reinterpret_cast<unsigned long long *>(base + list_bytes + 16 + slot_bytes - 16);
+        st = reinterpret_cast<RefineSlot *>(base + list_bytes);
+        counter = reinterpret_cast<unsigned long long *>(base + list_bytes + slot_bytes - 16);
     }
-    e = cudaMemsetAsync(listed, 0, sizeof(unsigned int), stream);
+    if (listing) e = cudaMemsetAsync(listed, 0, sizeof(unsigned int), stream);
     if (e == cudaSuccess && kDefer) e = cudaMemsetAsync(counter, 0, sizeof(unsigned long long), stream);
-    if (e == cudaSuccess) {
+    if (e == cudaSuccess && listing) {
         const int grid = grid_for(k_image_trivial<L>, d.nblocks, sms, 0, g_resident_trivial);
         k_image_trivial<L><<<grid, kWarpsPerCta * 32, 0, stream>>>(G, d, p, list, listed, kDefer ? st : nullptr);
         e = cudaGetLastError();
@@ -640,20 +654,18 @@ static cudaError_t launch_image_compacted(const GlobalTables *G, const ImageDesc
         e = cudaGetLastError();
     }
     if (e == cudaSuccess && kDefer) e = launch_refine(G, &d, nullptr, p, d.out, d.errors, st, d.nblocks, counter, stream, sms);
-    const cudaError_t f = scratch_free(scratch, stream);
+    const cudaError_t f = scratch ? scratch_free(scratch, stream) : cudaSuccess;
     return e != cudaSuccess ? e : f;
 }
 
-// Whether an image of `nblocks` blocks is encoded in one pass.  Two passes
-// keep blocks of 0 or 1 colours out of the searching warps, but cost a
-// scratch allocation, a memset and a second kernel that waits for the first.
-// One pass up to 512 blocks an SM (a block for every lane that fits), from
-// level 7 on, where a warp's search outweighs that, up to 96 (where the
-// CTA-wide pass begins).  One / two passes, us, no allocations by the caller:
-// level 4 at 64 x 64 17 / 32, 512 x 512 29 / 43, 1024 x 1024 37 / 49, 1448 x
-// 1448 64 / 59; level 6 27 / 41, 47 / 55, 65 / 69, 123 / 120; level 8 30 /
-// 43, 115 / 105 (at 384 x 384 84 / 88).
-static bool one_pass(int64_t nblocks, int sms) { return nblocks < (int64_t)sms * (L >= 7 ? 96 : 512); }
+// Whether an image of `nblocks` blocks is encoded in one pass of 4-warp CTAs.
+// Two passes keep blocks of 0 or 1 colours out of the searching warps, but
+// cost a scratch allocation, a memset and a second kernel that waits for the
+// first.  One pass below 96 blocks an SM, where the CTA-wide kernels begin;
+// at levels 2-3, which do not take those, up to 512.  One / two passes, us:
+// level 3 at 64 x 64 22 / 35, 1024 x 1024 33 / 40, 1448 x 1448 60 / 44; level
+// 6 27 / 41; level 8 30 / 43, 384 x 384 84 / 88, 512 x 512 115 / 105.
+static bool one_pass(int64_t nblocks, int sms) { return nblocks < (int64_t)sms * (L >= 4 ? 96 : 512); }
 
 static cudaError_t launch_image(const GlobalTables *G, const ImageDesc &d, const EncodeParams &p, cudaStream_t stream,
                                 int sms, RefineSlot *ext_st, unsigned long long *ext_counter) {

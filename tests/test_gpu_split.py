@@ -51,10 +51,11 @@ def test_cta_rounds(gpu_lib, level, bh):
     check(gpu_lib, img, level, 1, None)
 
 
-@pytest.mark.parametrize("level", (4, 8, 9))
-@pytest.mark.parametrize("bw,bh", ((14591, 1), (96, 152), (305, 255), (304, 256)))
+@pytest.mark.parametrize("level", (3, 4, 6, 8, 9))
+@pytest.mark.parametrize("bw,bh", ((14591, 1), (96, 152), (305, 255), (304, 256), (303, 452), (300, 456)))
 def test_cta_sizes(gpu_lib, level, bw, bh):
-    """Either side of 96 blocks an SM (8-warp CTAs from there) and of 512 (16-warp ones)."""
+    """Either side of 96 blocks an SM (8-warp CTAs from there), of 512 (16-warp ones, and at levels 2-5 a list of the
+    blocks to search) and of 900 (the list at levels 6-7)."""
     check(gpu_lib, synth.hard_mixture_image(4 * bw, 4 * bh, seed=bw + level), level, 1, None)
 
 
