@@ -1101,9 +1101,13 @@ __device__ __forceinline__ float encode_warp_ex(const WarpCtx &w, const Row &row
 
     if (active && O::cluster) count = reduce_colors(row, O::threshold, srow, any_black);
     // The SAT build unrolled no wider than the warp's largest colour count
-    // needs: 8, 12 or 16 entries (warp-uniform; levels 2-7, where most
-    // blocks reduce to a few colours; at levels 8-9 the extra builds' code
-    // cost 0.4%).
+    // needs: 8, 12 (levels 2-5) or 16 entries (warp-uniform; levels 2-7, where
+    // most blocks reduce to a few colours; at levels 8-9 the extra builds'
+    // code cost 0.4%).  Each width is 10-20 KB of straight-line code, so the
+    // 12-wide build, whose warps are few at levels 6-7, and narrow ones for
+    // the rarer rebuild without black colours cost more instruction fetches
+    // than they saved: without them 4096 x 4096 at level 7 927 -> 906 us, the
+    // hard mixture at level 6 2058 -> 1962.
     const int wmax = O::cluster && L <= 7 && !SIMD ? __reduce_max_sync(kFull, active ? count : 0) : 16;
     const int width = wmax <= 8 ? 8 : wmax <= 12 ? 12 : 16;
     // Float rows at levels 8-9, where the search is nearly all of the work,
@@ -1131,7 +1135,7 @@ __device__ __forceinline__ float encode_warp_ex(const WarpCtx &w, const Row &row
             }
             if (O::cluster) {
                 if (width == 8) build_sat_inplace<8>(srow, count, false);
-                else if (width == 12) build_sat_inplace<12>(srow, count, false);
+                else if (L <= 5 && width == 12) build_sat_inplace<12>(srow, count, false);
                 else build_sat_inplace(srow, count, false);
                 if (SIMD) fill_sat_tail(srow, count, p.simd_gather);
                 need4 = true;
@@ -1170,9 +1174,7 @@ __device__ __forceinline__ float encode_warp_ex(const WarpCtx &w, const Row &row
                     // then build the table of the non-black ones.
                     bool ab;
                     reduce_colors(row, O::threshold, srow, ab);
-                    count3 = width == 8    ? build_sat_inplace<8>(srow, count, true)
-                             : width == 12 ? build_sat_inplace<12>(srow, count, true)
-                                           : build_sat_inplace(srow, count, true);
+                    count3 = build_sat_inplace(srow, count, true);
                     if (SIMD) fill_sat_tail(srow, count3, p.simd_gather);
                     need3 = count3 > 0;
                 } else {
