@@ -30,6 +30,7 @@ struct ImageDesc {
     int vec16;  // rgba and pitch are 16-byte aligned: whole rows of a block load as one uint4
     int level, decoder, three_color_mode, three_color_black;
     float cw[3];
+    int overlapped;  // other launches of this call fill the SMs that this one leaves
 };
 
 // A warp's unit of batched work: per_task (at most 32) consecutive blocks of

@@ -317,8 +317,13 @@ template <int L, bool DEFER, int NW>
 __global__ void __launch_bounds__(NW * 32, 512 / (NW * 32))
     k_image_listed_cta(const GlobalTables *G, ImageDesc d, EncodeParams p, const uint32_t *list,
                        const unsigned int *listed, RefineSlot *st) {
-    const int64_t n = list ? (int64_t)*listed : d.nblocks;  // no list: every block of the image
-    const int per_cta = balanced_share(n, gridDim.x, 32 * NW, 1);
+    // Up to level 7: no list (one_cta_pass) means every block of the image, and
+    // a band of a larger image leaves its last round's SMs to the next band.
+    constexpr bool WHOLE = L <= 7;
+    const int64_t n = WHOLE && !list ? d.nblocks : (int64_t)*listed;
+    const int per_cta = WHOLE && d.overlapped && n > (int64_t)gridDim.x * 32 * NW
+                            ? 32 * NW
+                            : balanced_share(n, gridDim.x, 32 * NW, 1);
     const int64_t groups = (n + per_cta - 1) / per_cta;
     if ((int64_t)blockIdx.x >= groups) return;  // the whole CTA has no work
     extern __shared__ __align__(16) unsigned char smem[];
@@ -332,7 +337,7 @@ __global__ void __launch_bounds__(NW * 32, 512 / (NW * 32))
     for (int64_t grp = blockIdx.x; grp < groups; grp += gridDim.x) {
         const int64_t k = grp * per_cta + threadIdx.x;
         const bool active = (int)threadIdx.x < per_cta && k < n;
-        const int64_t b = !active ? 0 : list ? (int64_t)list[k] : k;
+        const int64_t b = !active ? 0 : WHOLE && !list ? k : (int64_t)list[k];
         __syncwarp();
         if (active) load_image_block_bytes(d, b, in + threadIdx.x * kInWordsByte);
         __syncwarp();
@@ -584,7 +589,7 @@ static int batch_cta_warps() {
 // 2048 x 2048 283 / 271.  At levels 8-9, where a CTA's blocks of 0 or 1
 // colours unbalance the searches, the list stays (level 8 at 1100 x 1100 274 /
 // 252).
-static bool one_cta_pass(int64_t nblocks, int sms) {
+static bool one_cta_pass(int64_t nblocks, int sms) {  // L <= 7: k_image_listed_cta's WHOLE
     return L >= 4 && L <= 7 && nblocks < (int64_t)sms * (L >= 6 ? 900 : 512);
 }
 

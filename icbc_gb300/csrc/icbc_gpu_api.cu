@@ -269,6 +269,7 @@ int resolve_image(const icbc_gpu_image &im, ImageDesc &d) {
     d.cw[0] = im.color_weights[0];
     d.cw[1] = im.color_weights[1];
     d.cw[2] = im.color_weights[2];
+    d.overlapped = 0;
     return ICBC_GPU_OK;
 }
 
@@ -495,11 +496,11 @@ int icbc_gpu_compress_bc1_image_simd(int simd_profile, const icbc_gpu_image *ima
     return e == cudaSuccess ? ICBC_GPU_OK : set_cuda_error(e);
 }
 
-int icbc_gpu_compress_bc1_image(const icbc_gpu_image *image, void *stream) {
-    if (!image) return ICBC_GPU_ERR_INVALID_ARGUMENT;
+static int compress_image(const icbc_gpu_image *image, void *stream, int overlapped) {
     ImageDesc d;
     int st = resolve_image(*image, d);
     if (st) return st;
+    d.overlapped = overlapped;
     cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
     const GlobalTables *G = nullptr;
     st = ensure_device_tables(&G);
@@ -507,6 +508,10 @@ int icbc_gpu_compress_bc1_image(const icbc_gpu_image *image, void *stream) {
     cudaError_t e = kImageLaunch[d.level](G, d, make_params(d.decoder, d.three_color_mode, d.three_color_black, d.cw),
                                           s, sm_count());
     return e == cudaSuccess ? ICBC_GPU_OK : set_cuda_error(e);
+}
+
+int icbc_gpu_compress_bc1_image(const icbc_gpu_image *image, void *stream) {
+    return image ? compress_image(image, stream, 0) : ICBC_GPU_ERR_INVALID_ARGUMENT;
 }
 
 int icbc_gpu_batch_create(const icbc_gpu_image *images, int n_images, icbc_gpu_batch **batch) {
@@ -884,15 +889,21 @@ int icbc_gpu_compress_bc1_image_host(const uint8_t *rgba, int32_t width, int32_t
         e = grow(reinterpret_cast<void **>(&H.d_plane), &H.plane_bytes, sizeof(float) * (size_t)width * height);
     if (e != cudaSuccess) return set_cuda_error(e);
     // Bands of whole block rows (each band is an independent image whose
-    // last band alone meets the bottom edge), at most kLevelBands[level] of
-    // at least 512 / that many block rows each.  The light levels take eight
-    // (their upload is most of the call, and eight bands overlap it with the
-    // encode); levels 6-7 four and 8-9 two: a band of an eighth of the image
-    // is too small for the listed pass's 16-warp CTAs and leaves a tail per
-    // band, and level 9's refinement queue needs many blocks per lane.
-    static const int kLevelBands[10] = {8, 8, 8, 8, 8, 8, 4, 4, 2, 2};
-    const int cap_bands = std::min(kMaxBands, kLevelBands[level < 0 ? 0 : level > 9 ? 9 : level]);
-    const int bands = (int)std::max<int64_t>(1, std::min<int64_t>(cap_bands, bh / (512 / cap_bands)));
+    // last band alone meets the bottom edge), at most kLevelBands[level] of at
+    // least kBandRows[level] block rows each: enough to overlap the upload, which is
+    // most of the light levels' call, with the encode, but each large enough
+    // for the encoder (level 9's refinement queue wants many blocks per lane).
+    // In us, against bands half as high, 4 from level 4 on (2 at levels 8-9):
+    // 2048 x 2048 at level 4 208 / 259, level 8 916 / 969; 1024 x 1024 at level
+    // 5 107 / 160; 4096 x 4096 at level 8 3321 / 3415.  Up to level 7 a band
+    // leaves its last round's SMs to the next one (levels 6-7 at 4096 x 4096
+    // 786 / 1073, evenly shared rounds 839 / 1091; at level 8 evenly shared
+    // ones are 5% faster).
+    static const int kLevelBands[10] = {8, 8, 8, 8, 5, 4, 4, 4, 3, 3};
+    static const int kBandRows[10] = {128, 128, 128, 128, 200, 128, 128, 128, 170, 170};
+    const int lv = level < 0 ? 0 : level > 9 ? 9 : level;
+    const int bands = (int)std::max<int64_t>(1, std::min<int64_t>(std::min(kMaxBands, kLevelBands[lv]),
+                                                                  bh / kBandRows[lv]));
     const int64_t rows_per = (bh + bands - 1) / bands;
     int st = ICBC_GPU_OK;
     for (int i = 0; i < bands && st == ICBC_GPU_OK; i++) {
@@ -934,7 +945,7 @@ int icbc_gpu_compress_bc1_image_host(const uint8_t *rgba, int32_t width, int32_t
         im.color_weights[2] = color_weights[2];
         im.out = static_cast<uint8_t *>(H.d_out) + 8 * b0;
         im.errors = errors ? H.d_err + b0 : nullptr;
-        st = icbc_gpu_compress_bc1_image(&im, cs);
+        st = compress_image(&im, cs, bands > 1 && level <= 7);
         if (st) break;
         e = cudaEventRecord(H.encoded[i], cs);
         if (e == cudaSuccess) e = cudaStreamWaitEvent(H.out, H.encoded[i], 0);
