@@ -58,7 +58,8 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32, 6)
             const ByteRow row{px, lut, d.weight_mode == ICBC_GPU_WEIGHTS_ALPHA};
             V3 c;
             int count;
-            other = !reduce_to_one(row, level_threshold(d.level), c, count);
+            other = d.level >= 8 ? !one_byte_colour(px, lut, row.alpha, c, count)
+                                 : !reduce_to_one(row, level_threshold(d.level), c, count);
             if (!other) {
                 EncodeParams p;
                 p.decoder = d.decoder;

@@ -198,7 +198,8 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32, 6) k_image_trivial(const Gl
             const ByteRow row{px, lut, alpha};
             V3 c;
             int count;
-            other = !reduce_to_one(row, Level<L>::threshold, c, count);
+            other = L >= 8 ? !one_byte_colour(px, lut, alpha, c, count)
+                           : !reduce_to_one(row, Level<L>::threshold, c, count);
             if (!other) {
                 uint32_t c0, c1, idx;
                 const float e = trivial_block<16>(D, lut, row, p, c, count, c0, c1, idx);
