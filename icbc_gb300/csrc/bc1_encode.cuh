@@ -117,24 +117,23 @@ __device__ __forceinline__ int reduce_colors(const Row &row, float threshold, fl
         const V3 ci = row.color(i);
         const float wi = row.weight(i);
         if (wi > 0) {
+            // The kept colour to merge with is found first, so that the lanes
+            // of a warp merge together, each with its own.
             int j = 0;
-            for (; j < n; j++) {
+            while (j < n && !near3(xyz(ld4(rrow + 4 * j)), ci, threshold)) j++;
+            if (j < n) {
                 const float4 c4 = ld4(rrow + 4 * j);
                 const V3 cj = xyz(c4);
-                if (near3(cj, ci, threshold)) {
-                    const float wj = c4.w;
-                    const float s = wj + wi;
-                    if (Row::kBounded)
-                        st4(rrow + 4 * j, make_float4(div_bounded(cj.x * wj + ci.x * wi, s),
-                                                      div_bounded(cj.y * wj + ci.y * wi, s),
-                                                      div_bounded(cj.z * wj + ci.z * wi, s), s));
-                    else
-                        st4(rrow + 4 * j, make_float4((cj.x * wj + ci.x * wi) / s, (cj.y * wj + ci.y * wi) / s,
-                                                      (cj.z * wj + ci.z * wi) / s, s));
-                    break;
-                }
-            }
-            if (j == n) {
+                const float wj = c4.w;
+                const float s = wj + wi;
+                if (Row::kBounded)
+                    st4(rrow + 4 * j, make_float4(div_bounded(cj.x * wj + ci.x * wi, s),
+                                                  div_bounded(cj.y * wj + ci.y * wi, s),
+                                                  div_bounded(cj.z * wj + ci.z * wi, s), s));
+                else
+                    st4(rrow + 4 * j, make_float4((cj.x * wj + ci.x * wi) / s, (cj.y * wj + ci.y * wi) / s,
+                                                  (cj.z * wj + ci.z * wi) / s, s));
+            } else {
                 st4(rrow + 4 * n, make_float4(ci.x, ci.y, ci.z, wi));
                 n++;
             }
