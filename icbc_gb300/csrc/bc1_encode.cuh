@@ -400,7 +400,7 @@ __device__ __forceinline__ bool optimize_end_points4(const Row &row, uint32_t in
 // `colors`: the reduced colours in a SAT row (SatColors) or a texel row.
 struct SatColors {
     static constexpr bool kBounded = false;
-    static constexpr int kUnroll = 1;
+    static constexpr int kBoxUnroll = 4;
     const float *p;
     __device__ __forceinline__ V3 color(int i) const { return xyz(ld4(p + 4 * i)); }
 };
@@ -409,7 +409,7 @@ template <class C>
 __device__ __forceinline__ void box_fit(const C &colors, int count, V3 &c0, V3 &c1) {
     c0 = v3(0.0f, 0.0f, 0.0f);
     c1 = v3(1.0f, 1.0f, 1.0f);
-#pragma unroll C::kUnroll
+#pragma unroll C::kBoxUnroll
     for (int i = 0; i < count; i++) {
         const V3 c = colors.color(i);
         if (C::kBounded) {  // no NaN and no -0: the reference's max and min are fmaxf and fminf
@@ -427,7 +427,7 @@ __device__ __forceinline__ void box_fit(const C &colors, int count, V3 &c0, V3 &
     c1 = saturate(c1 + inset);
     const V3 center = (c0 + c1) * 0.5f;
     float cov_xz = 0.0f, cov_yz = 0.0f;
-#pragma unroll C::kUnroll
+#pragma unroll C::kBoxUnroll
     for (int i = 0; i < count; i++) {
         const V3 t = colors.color(i) - center;
         cov_xz += t.x * t.z;

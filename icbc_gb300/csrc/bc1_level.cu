@@ -47,6 +47,7 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32) k_encode_blocks(const Globa
     SharedTables &T = *reinterpret_cast<SharedTables *>(smem);
     stage_tables(T, G);
     const WarpCtx w = warp_ctx<L>(smem, T, G, p.decoder);
+    if (L < 2) per_warp = 32;  // a constant: these kernels take microseconds
     const int64_t groups = (n + per_warp - 1) / per_warp;
     for (int64_t g = (int64_t)blockIdx.x * kWarpsPerCta + (threadIdx.x >> 5); g < groups;
          g += (int64_t)gridDim.x * kWarpsPerCta) {
@@ -92,6 +93,7 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32) k_encode_image(const Global
         stage_tables(T, G);
         w = warp_ctx<L>(smem, T, G, p.decoder);
     }
+    if (L < 2) per_warp = 32;
     const int64_t groups = (d.nblocks + per_warp - 1) / per_warp;
     for (int64_t g = (int64_t)blockIdx.x * kWarpsPerCta + (threadIdx.x >> 5); g < groups;
          g += (int64_t)gridDim.x * kWarpsPerCta) {
