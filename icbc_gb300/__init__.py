@@ -650,7 +650,8 @@ def set_launch_config(level: int, groups_per_warp: int, persistent: int, cta_war
 
 
 def get_batch_cta_warps(level: int) -> int:
-    """The batched form's CTA size at a level (0: the default, 8 from level 4 on, else 4)."""
+    """The batched form's CTA size at a level (0: the default, 4 or 8 by the
+    batch's levels and block counts)."""
     c = LaunchConfig()
     _check(load().icbc_gpu_get_launch_config(int(level), ctypes.byref(c)), "get_launch_config")
     return c.batch_cta_warps

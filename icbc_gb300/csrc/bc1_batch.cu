@@ -21,10 +21,10 @@ constexpr bool kBytes = ICBC_BATCH_BYTES != 0;
 template <bool BYTES>
 __global__ void __launch_bounds__(kWarpsPerCta * 32, BYTES ? 4 : 1)
     k_encode_batch(const GlobalTables *G, const ImageDesc *images, const BatchTask *tasks, const uint32_t *task_start,
-                   int n_images, int ntasks, int per_task, int *counter, const int64_t *refine_base, RefineSlot *slots,
+                   int n_images, int ntasks, int *counter, const int64_t *refine_base, RefineSlot *slots,
                    BatchLists lists) {
     extern __shared__ __align__(16) unsigned char smem[];
-    run_batch<BYTES, -1>(G, smem, images, tasks, task_start, n_images, 0, ntasks, per_task, counter, refine_base, slots, lists);
+    run_batch<BYTES, -1>(G, smem, images, tasks, task_start, n_images, 0, ntasks, counter, refine_base, slots, lists);
 }
 
 #if ICBC_BATCH_BYTES
@@ -37,19 +37,18 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32, BYTES ? 4 : 1)
 // table is in shared memory, so six CTAs fit on an SM.
 __global__ void __launch_bounds__(kWarpsPerCta * 32, 6)
     k_batch_trivial(const GlobalTables *G, const ImageDesc *images, const BatchTask *tasks, const uint32_t *task_start,
-                    int n_images, int ntasks, int per_task, BatchLists lists, const int64_t *refine_base,
-                    RefineSlot *slots) {
+                    int n_images, int ntasks, BatchLists lists, const int64_t *refine_base, RefineSlot *slots) {
     __shared__ float lut[256];
     for (int i = threadIdx.x; i < 256; i += blockDim.x) lut[i] = G->s.lut255[i];
     __syncthreads();
     const int lane = threadIdx.x & 31;
     for (int t = blockIdx.x * kWarpsPerCta + (threadIdx.x >> 5); t < ntasks; t += gridDim.x * kWarpsPerCta) {
-        const BatchTask task = batch_task(tasks, task_start, n_images, t, per_task);
+        const BatchTask task = batch_task(tasks, task_start, n_images, t);
         const int64_t lb = lists.list_base[task.image];
         if (lb < 0) continue;
         const ImageDesc &d = images[task.image];
         const int64_t b = (int64_t)task.first_block + lane;
-        const bool active = lane < per_task && b < d.nblocks;
+        const bool active = lane < (int)task.blocks && b < d.nblocks;
         const int64_t sb = (d.level == 9 && refine_base) ? refine_base[task.image] : -1;
         bool other = false;
         if (active) {
@@ -98,15 +97,15 @@ static int batch_trivial_resident() {
 void prepare_batch_trivial() { batch_trivial_resident(); }
 
 cudaError_t launch_batch_trivial(const GlobalTables *G, const ImageDesc *images, const BatchTask *tasks,
-                                 const uint32_t *task_start, int n_images, int ntasks, int per_task, BatchLists lists,
+                                 const uint32_t *task_start, int n_images, int ntasks, BatchLists lists,
                                  const int64_t *refine_base, RefineSlot *slots, cudaStream_t stream, int sms) {
     if (ntasks <= 0) return cudaSuccess;
     const int resident = batch_trivial_resident();
     const int64_t need = ((int64_t)ntasks + kWarpsPerCta - 1) / kWarpsPerCta;
     const int64_t cap = (int64_t)sms * resident;
     const int grid = (int)(need < cap ? need : cap);
-    k_batch_trivial<<<grid, kWarpsPerCta * 32, 0, stream>>>(G, images, tasks, task_start, n_images, ntasks, per_task,
-                                                            lists, refine_base, slots);
+    k_batch_trivial<<<grid, kWarpsPerCta * 32, 0, stream>>>(G, images, tasks, task_start, n_images, ntasks, lists,
+                                                            refine_base, slots);
     return cudaGetLastError();
 }
 #endif
@@ -122,14 +121,14 @@ cudaError_t launch_batch_trivial(const GlobalTables *G, const ImageDesc *images,
 static size_t batch_smem() { return kBytes ? smem_bytes_byte_rows() : smem_bytes(true); }
 
 cudaError_t ICBC_BATCH_FN(launch_encode_batch)(const GlobalTables *G, const ImageDesc *images, const BatchTask *tasks,
-                                               const uint32_t *task_start, int n_images, int ntasks, int per_task,
-                                               int *counter, cudaStream_t stream, int grid, const int64_t *refine_base,
+                                               const uint32_t *task_start, int n_images, int ntasks, int *counter,
+                                               cudaStream_t stream, int grid, const int64_t *refine_base,
                                                RefineSlot *slots, BatchLists lists) {
     const size_t smem = batch_smem();
     cudaError_t e = cudaFuncSetAttribute(k_encode_batch<kBytes>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     k_encode_batch<kBytes><<<grid, kWarpsPerCta * 32, smem, stream>>>(G, images, tasks, task_start, n_images, ntasks,
-                                                                       per_task, counter, refine_base, slots, lists);
+                                                                       counter, refine_base, slots, lists);
     return cudaGetLastError();
 }
 

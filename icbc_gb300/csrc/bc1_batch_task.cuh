@@ -7,12 +7,17 @@
 
 namespace icbc_gpu {
 
-// Task t of a batch: an entry of the explicit list, or -- without one --
-// found from per-image offsets: task t belongs to the last image whose first
+__device__ __forceinline__ BatchTask load_task(const BatchTask *t) {
+    const uint4 v = *reinterpret_cast<const uint4 *>(t);
+    return BatchTask{v.x, v.y, v.z, v.w};
+}
+
+// Task t of a batch: an entry of the explicit list, or -- without one, tasks
+// of 32 blocks -- found from per-image offsets: task t belongs to the last image whose first
 // task (`task_start[i]`, n_images + 1 entries) is <= t.
 __device__ __forceinline__ BatchTask batch_task(const BatchTask *tasks, const uint32_t *task_start, int n_images,
-                                                int t, int per_task) {
-    if (tasks) return tasks[t];
+                                                int t) {
+    if (tasks) return load_task(tasks + t);
     int lo = 0, hi = n_images;
     while (hi - lo > 1) {
         const int mid = (lo + hi) >> 1;
@@ -21,7 +26,8 @@ __device__ __forceinline__ BatchTask batch_task(const BatchTask *tasks, const ui
     }
     BatchTask task;
     task.image = (uint32_t)lo;
-    task.first_block = (uint32_t)(t - (int)task_start[lo]) * (uint32_t)per_task;
+    task.first_block = (uint32_t)(t - (int)task_start[lo]) * 32u;
+    task.blocks = 32u;
     return task;
 }
 
@@ -74,12 +80,12 @@ __device__ __forceinline__ float encode_task_at(int level, bool defer, const War
 // plain level-9 launches, so lanes do not wait for each other's refinement.
 // With `lists.list` (second pass of a two-pass batch), the tasks of an image
 // with list_base >= 0 cover the image's list instead of its blocks: task
-// blocks first_block .. first_block + per_task - 1 are list entries, and tasks past
-// the list's end have nothing to do.
+// blocks first_block .. first_block + blocks - 1 are list entries, and tasks
+// past the list's end have nothing to do.
 template <bool BYTES, int L>
 __device__ __forceinline__ void run_batch(const GlobalTables *G, unsigned char *smem, const ImageDesc *images,
                                           const BatchTask *tasks, const uint32_t *task_start, int n_images, int task0,
-                                          int ntasks, int per_task, int *counter, const int64_t *refine_base, RefineSlot *slots,
+                                          int ntasks, int *counter, const int64_t *refine_base, RefineSlot *slots,
                                           BatchLists lists) {
     SharedTables &T = *reinterpret_cast<SharedTables *>(smem);
     stage_tables(T, G);
@@ -89,16 +95,16 @@ __device__ __forceinline__ void run_batch(const GlobalTables *G, unsigned char *
         if (lane == 0) t = atomicAdd(counter, 1);
         t = __shfl_sync(kFull, t, 0);
         if (t >= ntasks) break;
-        const BatchTask task = batch_task(tasks, task_start, n_images, task0 + t, per_task);
+        const BatchTask task = batch_task(tasks, task_start, n_images, task0 + t);
         const ImageDesc &d = images[task.image];
         const int level = L >= 0 ? L : d.level;
         const int64_t lb = lists.list ? lists.list_base[task.image] : -1;
         int64_t b = (int64_t)task.first_block + lane;
-        bool active = lane < per_task && b < d.nblocks;
+        bool active = lane < (int)task.blocks && b < d.nblocks;
         if (lb >= 0) {
             const int64_t n = lists.listed[task.image];
             if ((int64_t)task.first_block >= n) continue;  // the whole task was finished by the first pass
-            active = lane < per_task && b < n;
+            active = lane < (int)task.blocks && b < n;
             b = active ? (int64_t)lists.list[lb + b] : 0;
         }
         EncodeParams p;

@@ -6,6 +6,7 @@
 
 #include "../../include/icbc_gpu.h"
 #include "bc1_encode.cuh"
+#include "bc1_shares.h"
 
 namespace icbc_gpu {
 
@@ -33,11 +34,13 @@ struct ImageDesc {
     int overlapped;  // other launches of this call fill the SMs that this one leaves
 };
 
-// A warp's unit of batched work: per_task (at most 32) consecutive blocks of
-// one image, the same number for every task of a batch.
-struct BatchTask {
+// A warp's unit of batched work: `blocks` (at most 32) consecutive blocks of
+// one image (fewer at its end).  One 16-byte load.
+struct alignas(16) BatchTask {
     uint32_t image;
     uint32_t first_block;
+    uint32_t blocks;
+    uint32_t unused;
 };
 
 using BlocksLauncher = cudaError_t (*)(const GlobalTables *, const BlocksSrc &, const EncodeParams &, void *, float *,
@@ -83,7 +86,7 @@ using BatchLevelLauncher = cudaError_t (*)(const GlobalTables *, const ImageDesc
                                            int *, cudaStream_t, int, const int64_t *, RefineSlot *, BatchLists);
 #define ICBC_DECLARE_BATCH_LEVEL(L)                                                                                \
     cudaError_t launch_batch_level_l##L(const GlobalTables *G, const ImageDesc *images, const BatchTask *tasks,     \
-                                        int task0, int ntasks, int per_task, int *counter, cudaStream_t stream, int grid, \
+                                        int task0, int ntasks, int planned_warps, int *counter, cudaStream_t stream, int grid, \
                                         const int64_t *refine_base, RefineSlot *slots, BatchLists lists);
 ICBC_DECLARE_BATCH_LEVEL(0)
 ICBC_DECLARE_BATCH_LEVEL(1)
@@ -101,23 +104,23 @@ ICBC_DECLARE_BATCH_LEVEL(9)
 // weight plane), four CTAs per SM; else float rows.  With lists.list, the
 // tasks of listed images take their blocks from the lists.
 cudaError_t launch_encode_batch_float(const GlobalTables *G, const ImageDesc *images, const BatchTask *tasks,
-                                      const uint32_t *task_start, int n_images, int ntasks, int per_task, int *counter,
+                                      const uint32_t *task_start, int n_images, int ntasks, int *counter,
                                       cudaStream_t stream, int grid, const int64_t *refine_base, RefineSlot *slots,
                                       BatchLists lists);
 cudaError_t launch_encode_batch_bytes(const GlobalTables *G, const ImageDesc *images, const BatchTask *tasks,
-                                      const uint32_t *task_start, int n_images, int ntasks, int per_task, int *counter,
+                                      const uint32_t *task_start, int n_images, int ntasks, int *counter,
                                       cudaStream_t stream, int grid, const int64_t *refine_base, RefineSlot *slots,
                                       BatchLists lists);
 int batch_ctas_per_sm_float();
 int batch_ctas_per_sm_bytes();
 inline cudaError_t launch_encode_batch(const GlobalTables *G, const ImageDesc *images, const BatchTask *tasks,
-                                       const uint32_t *task_start, int n_images, int ntasks, int per_task, int *counter,
+                                       const uint32_t *task_start, int n_images, int ntasks, int *counter,
                                        cudaStream_t stream, int grid, const int64_t *refine_base = nullptr,
                                        RefineSlot *slots = nullptr, bool byte_rows = false,
                                        BatchLists lists = BatchLists{nullptr, nullptr, nullptr}) {
-    return byte_rows ? launch_encode_batch_bytes(G, images, tasks, task_start, n_images, ntasks, per_task, counter, stream, grid,
+    return byte_rows ? launch_encode_batch_bytes(G, images, tasks, task_start, n_images, ntasks, counter, stream, grid,
                                                  refine_base, slots, lists)
-                     : launch_encode_batch_float(G, images, tasks, task_start, n_images, ntasks, per_task, counter, stream, grid,
+                     : launch_encode_batch_float(G, images, tasks, task_start, n_images, ntasks, counter, stream, grid,
                                                  refine_base, slots, lists);
 }
 // First pass of a two-pass batch (byte rows): finishes the blocks of 0 or 1
@@ -125,7 +128,7 @@ inline cudaError_t launch_encode_batch(const GlobalTables *G, const ImageDesc *i
 // empty refinement slot) and lists the rest.  A grid stride over the first
 // ntasks tasks (`tasks`, or per-image offsets as for launch_encode_batch).
 cudaError_t launch_batch_trivial(const GlobalTables *G, const ImageDesc *images, const BatchTask *tasks,
-                                 const uint32_t *task_start, int n_images, int ntasks, int per_task, BatchLists lists,
+                                 const uint32_t *task_start, int n_images, int ntasks, BatchLists lists,
                                  const int64_t *refine_base, RefineSlot *slots, cudaStream_t stream, int sms);
 // Loads launch_batch_trivial's kernel (which otherwise loads on its first launch).
 void prepare_batch_trivial();
@@ -163,10 +166,6 @@ cudaError_t launch_refine_batch(const GlobalTables *G, const ImageDesc *images, 
 // or float blocks (`blocks`), p.simd_* set.
 cudaError_t launch_simd(const GlobalTables *G, const ImageDesc *image, const BlocksSrc *blocks, const EncodeParams &p,
                         uint2 *out, float *errors, int64_t n, int level, cudaStream_t stream);
-
-// Blocks a batched task takes, for `blocks` in all: 32, or as few as give
-// every resident warp one.
-int batch_task_blocks(int64_t blocks);
 
 // Launch shape of the plain kernels of a level (autotuned or default).
 struct LaunchShape {

@@ -17,26 +17,6 @@ namespace icbc_gpu {
 
 // ------------------------------------------------------------- kernels --
 
-// How many of n blocks a worker (a warp of 32 lanes, or a CTA) takes at a
-// time when `workers` share them: as few as the rounds they need anyway allow,
-// at most `most`.  A last round that is nearly empty costs as much as a full
-// one, and an image too small for 32 blocks a warp leaves most SMs without a
-// warp while the others run long ones (the cluster search spreads a warp's
-// blocks over its 32 lanes however many they are).  Against 32 blocks a warp
-// always, in us: level 8 at 64 x 64 187 -> 48, 512 x 512 194 -> 116, 2048 x
-// 2048 (the 16-warp CTAs' last round) 1018 -> 826, 4096 x 4096 3342 -> 3114;
-// with a weight plane 1000 x 600 431 -> 237; 40,000 float blocks 303 -> 155.
-// A warp takes at least `least` blocks: below level 4, where the search is a
-// small part of a block's work, warps with few blocks only add lanes without
-// one (level 3 at 1024 x 1024: 45 us with 16, 51 with 1; level 7 at 64 x 64:
-// 79 with 16, 48 with 1).
-__host__ __device__ constexpr int balanced_share(int64_t n, int64_t workers, int most, int least) {
-    const int64_t rounds = (n + workers * most - 1) / (workers * most);
-    const int64_t share = rounds < 1 ? 1 : (n + workers * rounds - 1) / (workers * rounds);
-    return (int)(share < least ? least : share);
-}
-__host__ __device__ constexpr int least_per_warp(int level) { return level >= 4 ? 1 : 16; }
-
 // With DEFER (level 9 only) refinement is left to k_refine: the kernel
 // records each block's starting error and whether refinement applies.
 template <int L, bool DEFER>
@@ -373,7 +353,7 @@ __global__ void __launch_bounds__(NW * 32, 512 / (NW * 32))
 template <int LV, int NW>
 __global__ void __launch_bounds__(NW * 32, 512 / (NW * 32))
     k_batch_level_cta(const GlobalTables *G, const ImageDesc *images, const BatchTask *tasks, int task0, int ntasks,
-                      int per_task, int *counter, const int64_t *refine_base, RefineSlot *slots, BatchLists lists) {
+                      int *counter, const int64_t *refine_base, RefineSlot *slots, BatchLists lists) {
     extern __shared__ __align__(16) unsigned char smem[];
     SharedTables &T = *reinterpret_cast<SharedTables *>(smem);
     stage_tables(T, G);
@@ -415,14 +395,14 @@ __global__ void __launch_bounds__(NW * 32, 512 / (NW * 32))
         const int have = round[NW];
         if (have == 0) break;
         const bool has_task = warp < have;
-        const BatchTask task = has_task ? tasks[task0 + round[warp]] : BatchTask{0u, 0u};
+        const BatchTask task = has_task ? load_task(tasks + task0 + round[warp]) : BatchTask{};
         const ImageDesc &d = images[task.image];
         const int64_t lb = lists.list ? lists.list_base[task.image] : -1;
         int64_t b = (int64_t)task.first_block + lane;
-        bool active = has_task && lane < per_task && b < d.nblocks;
+        bool active = has_task && lane < (int)task.blocks && b < d.nblocks;
         if (has_task && lb >= 0) {
             const int64_t n = lists.listed[task.image];
-            active = lane < per_task && b < n;  // tasks past the list's end: finished by the first pass
+            active = lane < (int)task.blocks && b < n;  // tasks past the list's end: finished by the first pass
             b = active ? (int64_t)lists.list[lb + b] : 0;
         }
         if (lane == 0)
@@ -476,9 +456,9 @@ __global__ void __launch_bounds__(NW * 32, 512 / (NW * 32))
 template <int LV>
 __global__ void __launch_bounds__(kWarpsPerCta * 32, 4)
     k_batch_level(const GlobalTables *G, const ImageDesc *images, const BatchTask *tasks, int task0, int ntasks,
-                  int per_task, int *counter, const int64_t *refine_base, RefineSlot *slots, BatchLists lists) {
+                  int *counter, const int64_t *refine_base, RefineSlot *slots, BatchLists lists) {
     extern __shared__ __align__(16) unsigned char smem[];
-    run_batch<true, LV>(G, smem, images, tasks, nullptr, 0, task0, ntasks, per_task, counter, refine_base, slots, lists);
+    run_batch<true, LV>(G, smem, images, tasks, nullptr, 0, task0, ntasks, counter, refine_base, slots, lists);
 }
 
 constexpr int L = ICBC_LEVEL;
@@ -597,14 +577,14 @@ static int listed_cta_warps(int64_t nblocks, int sms) {
     return c > 4 && nblocks >= (int64_t)sms * 96 ? 8 : 4;
 }
 
-// The batched form's per-level kernel's CTA size: the launch shape's, else 8
-// from level 4 on, where the CTA's stages in step keep the long per-block code
-// in the instruction cache (300 images of 64 to 2048 a side, all levels: 7.21
-// ms with 4-warp CTAs, 6.23 with 8, 6.43 with 16; 400 of the mixed batch 6.53
-// / 6.34 / 6.45; below level 4 either size takes the same time).
-static int batch_cta_warps() {
+// The batched form's per-level kernel's CTA size: the launch shape's, else the
+// batch's plan (batch_shape): 8 where the CTA's stages in step keep the long
+// per-block code in the instruction cache (300 images of 64 to 2048 a side,
+// all levels: 7.21 ms with 4-warp CTAs, 6.23 with 8, 6.43 with 16; 400 of the
+// mixed batch 6.53 / 6.34 / 6.45).
+static int batch_cta_warps(int planned) {
     const int c = launch_shape(L).batch_cta_warps;
-    return c == 4 || c == 8 || c == 16 ? c : L >= 4 ? 8 : 4;
+    return c == 4 || c == 8 || c == 16 ? c : planned;
 }
 
 // Whether the CTA-wide pass takes all of an image's blocks instead of a list,
@@ -731,11 +711,11 @@ cudaError_t ICBC_CAT(launch_blocks_l, ICBC_LEVEL)(const GlobalTables *G, const B
 }
 
 cudaError_t ICBC_CAT(launch_batch_level_l, ICBC_LEVEL)(const GlobalTables *G, const ImageDesc *images,
-                                                        const BatchTask *tasks, int task0, int ntasks, int per_task,
+                                                        const BatchTask *tasks, int task0, int ntasks, int planned_warps,
                                                         int *counter, cudaStream_t stream, int grid, const int64_t *refine_base,
                                                         RefineSlot *slots, BatchLists lists) {
     // `grid` counts 4-warp CTAs; a CTA-wide kernel gets as many warps in all.
-    const int cta_warps = Level<L>::cluster && (L < 9 || refine_base) ? batch_cta_warps() : 4;
+    const int cta_warps = Level<L>::cluster && (L < 9 || refine_base) ? batch_cta_warps(planned_warps) : 4;
     if (cta_warps != 4) {
         const size_t smem = cta_warps == 16 ? batch_smem_bytes<16>() : batch_smem_bytes<8>();
         int *resident = cta_warps == 16 ? &g_resident_batch16 : &g_resident_batch8;
@@ -745,17 +725,17 @@ cudaError_t ICBC_CAT(launch_batch_level_l, ICBC_LEVEL)(const GlobalTables *G, co
         const int want = (grid * kWarpsPerCta + cta_warps - 1) / cta_warps;
         const int ctas = std::max(1, std::min(want, current_sm_count() * *resident));
         if (cta_warps == 16)
-            k_batch_level_cta<L, 16><<<ctas, 16 * 32, smem, stream>>>(G, images, tasks, task0, ntasks, per_task, counter,
+            k_batch_level_cta<L, 16><<<ctas, 16 * 32, smem, stream>>>(G, images, tasks, task0, ntasks, counter,
                                                                        refine_base, slots, lists);
         else
-            k_batch_level_cta<L, 8><<<ctas, 8 * 32, smem, stream>>>(G, images, tasks, task0, ntasks, per_task, counter,
+            k_batch_level_cta<L, 8><<<ctas, 8 * 32, smem, stream>>>(G, images, tasks, task0, ntasks, counter,
                                                                      refine_base, slots, lists);
         return cudaGetLastError();
     }
     const size_t smem = smem_bytes_byte_rows();
     cudaError_t e = cudaFuncSetAttribute(k_batch_level<L>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    k_batch_level<L><<<grid, kWarpsPerCta * 32, smem, stream>>>(G, images, tasks, task0, ntasks, per_task, counter, refine_base,
+    k_batch_level<L><<<grid, kWarpsPerCta * 32, smem, stream>>>(G, images, tasks, task0, ntasks, counter, refine_base,
                                                                slots, lists);
     return cudaGetLastError();
 }

@@ -295,15 +295,6 @@ int ensure_tables_on_device(const GlobalTables **out) { return ensure_device_tab
 
 int current_sm_count() { return sm_count(); }
 
-// A small batch in tasks of 32 blocks would leave most warps without one, and
-// a warp's time grows with its blocks: it takes tasks of as few blocks as give
-// each of the resident warps (16 an SM) one (10 images of up to 256 x 256:
-// 169 -> 84 us with the 8-warp CTAs; 30 of up to 512 x 512: 410 -> 371).
-int batch_task_blocks(int64_t blocks) {
-    const int64_t warps = 16 * (int64_t)sm_count();
-    return (int)std::max<int64_t>(1, std::min<int64_t>(32, (blocks + warps - 1) / warps));
-}
-
 }  // namespace icbc_gpu
 
 // Relative cost of a 32-block task per level, used to order batched work
@@ -549,18 +540,30 @@ int icbc_gpu_batch_create(const icbc_gpu_image *images, int n_images, icbc_gpu_b
         if (ka != kb) return ka < kb;
         return descs[a].nblocks > descs[b].nblocks;
     });
+    // Byte texel rows (four CTAs per SM) unless an image brings a weight plane
+    // (three).
+    bool byte_rows = true;
+    for (int i = 0; i < n_images; i++) byte_rows &= descs[i].weight_mode != ICBC_GPU_WEIGHTS_PLANE;
+    const int grid = sm_count() * batch_ctas_per_sm(byte_rows);
     std::vector<int> own;  // images that get their level's own launch
     std::vector<BatchTask> tasks;
-    int64_t shared_blocks = 0;
-    for (int i : order)
-        if (descs[i].nblocks < kOwnLaunchBlocks) shared_blocks += descs[i].nblocks;
-    const int per_task = batch_task_blocks(shared_blocks);
+    std::vector<int> levels;
+    std::vector<int64_t> counts;
+    for (int i : order) {
+        if (descs[i].nblocks >= kOwnLaunchBlocks) continue;
+        levels.push_back(descs[i].level);
+        counts.push_back(descs[i].nblocks);
+    }
+    const BatchShape shape = batch_shape(levels.data(), counts.data(), (int)levels.size(),
+                                         (int64_t)grid * kWarpsPerCta, byte_rows);
     for (int i : order) {
         if (descs[i].nblocks >= kOwnLaunchBlocks) {
             own.push_back(i);
             continue;
         }
-        for (int64_t b = 0; b < descs[i].nblocks; b += per_task) tasks.push_back(BatchTask{(uint32_t)i, (uint32_t)b});
+        const int step = shape.task_blocks[descs[i].level];
+        for (int64_t b = 0; b < descs[i].nblocks; b += step)
+            tasks.push_back(BatchTask{(uint32_t)i, (uint32_t)b, (uint32_t)step, 0u});
     }
     if (tasks.size() > 0x7fffffff) return ICBC_GPU_ERR_INVALID_ARGUMENT;
     // Refinement slots of the level-9 images, in task order; then those of
@@ -583,10 +586,7 @@ int icbc_gpu_batch_create(const icbc_gpu_image *images, int n_images, icbc_gpu_b
     }
     icbc_gpu_batch *B = new icbc_gpu_batch();
     B->ntasks = (int)tasks.size();
-    // Byte texel rows (four CTAs per SM) unless an image brings a weight plane.
-    bool byte_rows = true;
-    for (int i = 0; i < n_images; i++) byte_rows &= descs[i].weight_mode != ICBC_GPU_WEIGHTS_PLANE;
-    B->grid = sm_count() * batch_ctas_per_sm(byte_rows);
+    B->grid = grid;
     B->refine_total = refine_total;
     B->map_n = (int)map_image.size();
     // Byte-row batches run in two passes: the blocks of 0 or 1 reduced
@@ -676,7 +676,7 @@ int icbc_gpu_batch_create(const icbc_gpu_image *images, int n_images, icbc_gpu_b
         if (e1 == cudaSuccess && B->d_list) {
             e1 = cudaMemsetAsync(B->d_listed, 0, sizeof(unsigned int) * n_images, cs);
             if (e1 == cudaSuccess)
-                e1 = launch_batch_trivial(G, B->d_images, B->d_tasks, nullptr, n_images, B->ntasks_listed, per_task, lists,
+                e1 = launch_batch_trivial(G, B->d_images, B->d_tasks, nullptr, n_images, B->ntasks_listed, lists,
                                           B->d_refine_base, B->d_slots, cs, sm_count());
         }
         cudaError_t e2 = e1;
@@ -688,13 +688,13 @@ int icbc_gpu_batch_create(const icbc_gpu_image *images, int n_images, icbc_gpu_b
                 const int grid = std::min(B->grid, (n + kWarpsPerCta - 1) / kWarpsPerCta);  // a task per warp at most
                 e2 = cudaStreamWaitEvent(lv_stream[l], fork, 0);
                 if (e2 == cudaSuccess)
-                    e2 = kBatchLevelLaunch[l](G, B->d_images, B->d_tasks, lv_begin[l], n, per_task, B->d_counter + 1 + l,
+                    e2 = kBatchLevelLaunch[l](G, B->d_images, B->d_tasks, lv_begin[l], n, shape.cta_warps[l], B->d_counter + 1 + l,
                                               lv_stream[l], grid, B->d_refine_base, B->d_slots, lists);
                 if (e2 == cudaSuccess) e2 = cudaEventRecord(lv_done[l], lv_stream[l]);
                 if (e2 == cudaSuccess) e2 = cudaStreamWaitEvent(cs, lv_done[l], 0);
             }
         } else if (e2 == cudaSuccess && B->ntasks) {
-            e2 = launch_encode_batch(G, B->d_images, B->d_tasks, nullptr, n_images, B->ntasks, per_task, B->d_counter, cs,
+            e2 = launch_encode_batch(G, B->d_images, B->d_tasks, nullptr, n_images, B->ntasks, B->d_counter, cs,
                                      B->grid, B->d_refine_base, B->d_slots, byte_rows, lists);
         }
         if (e2 == cudaSuccess && refine_total) {

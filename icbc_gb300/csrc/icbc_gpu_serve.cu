@@ -210,7 +210,7 @@ int launch_slot(icbc_gpu_server *S, Slot &slot) {
     // small request sooner (mean 0.19 -> 0.18 ms at 500 requests/s) but take
     // more of the GPU from the other launches in flight (mean 0.59 -> 0.66 ms
     // at 20,000, p99 6.0 -> 7.6 ms at saturation).
-    constexpr uint32_t per_task = 32;
+    constexpr int kTaskBlocks = 32;  // batch_task's
     uint32_t total = 0, listed_tasks = 0;  // level-2..9 requests come first: their tasks lead
     for (size_t i = 0; i < reqs.size() && e == cudaSuccess; i++) {
         Request *q = reqs[i];
@@ -231,8 +231,8 @@ int launch_slot(icbc_gpu_server *S, Slot &slot) {
         slot.h_images[i] = d;
         slot.h_start[i] = total;
         slot.h_list_base[i] = d.level >= 2 && d.nblocks > 0 ? (int64_t)((q->dev_off + q->list_off) / 4) : -1;
-        if (d.level >= 2) listed_tasks = total + (uint32_t)((d.nblocks + per_task - 1) / per_task);
-        total += (uint32_t)((d.nblocks + per_task - 1) / per_task);
+        if (d.level >= 2) listed_tasks = total + (uint32_t)((d.nblocks + kTaskBlocks - 1) / kTaskBlocks);
+        total += (uint32_t)((d.nblocks + kTaskBlocks - 1) / kTaskBlocks);
     }
     slot.h_start[reqs.size()] = total;
     const int n = (int)reqs.size();
@@ -248,8 +248,8 @@ int launch_slot(icbc_gpu_server *S, Slot &slot) {
                             slot.stream);
         if (e == cudaSuccess) e = cudaMemsetAsync(slot.d_listed, 0, sizeof(unsigned int) * n, slot.stream);
         if (e == cudaSuccess)
-            e = launch_batch_trivial(S->G, slot.d_images, nullptr, slot.d_start, n, (int)listed_tasks, (int)per_task, lists, nullptr,
-                                     nullptr, slot.stream, current_sm_count());
+            e = launch_batch_trivial(S->G, slot.d_images, nullptr, slot.d_start, n, (int)listed_tasks, lists, nullptr, nullptr,
+                                     slot.stream, current_sm_count());
     }
     if (e == cudaSuccess) {
         // A persistent grid no larger than the batch's work (four tasks per
@@ -260,7 +260,7 @@ int launch_slot(icbc_gpu_server *S, Slot &slot) {
         // 20,000 requests/s 2.6-3.2 ms instead of 3.2-10 ms).
         // Requests carry uniform or alpha weights: the byte-row kernel.
         const uint32_t cap = total > (uint32_t)S->grid ? (uint32_t)S->grid * 3 / 4 : (uint32_t)S->grid;
-        e = launch_encode_batch(S->G, slot.d_images, nullptr, slot.d_start, n, (int)total, (int)per_task, slot.d_counter,
+        e = launch_encode_batch(S->G, slot.d_images, nullptr, slot.d_start, n, (int)total, slot.d_counter,
                                 slot.stream, (int)std::min<uint32_t>(cap, (total + 3) / 4), nullptr, nullptr, true,
                                 listed_tasks ? lists : BatchLists{nullptr, nullptr, nullptr});
     }

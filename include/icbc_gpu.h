@@ -359,13 +359,13 @@ int icbc_gpu_compress_bc1_mips(const icbc_gpu_image *image, int32_t levels, void
  * takes 4); 0 = the level's default.  An image too small to give every
  * resident warp 32 blocks takes smaller shares whatever the shape.  Defaults:
  * 1 / persistent at levels 0-1, 2 / not persistent at levels 2-9, cta_warps
- * 16 and batch_cta_warps 8 from level 4 on (else 4).  Not for use while
- * launches run or batches are created. */
+ * 16 from level 4 on (else 4), batch_cta_warps 4 or 8 by the batch's levels
+ * and block counts.  Not for use while launches run or batches are created. */
 typedef struct icbc_gpu_launch_config {
     int32_t groups_per_warp;
     int32_t persistent;
     int32_t cta_warps;
-    int32_t batch_cta_warps;  /* 0 = the default: 8 from level 4 on, else 4 */
+    int32_t batch_cta_warps;
 } icbc_gpu_launch_config;
 int icbc_gpu_set_launch_config(int level, const icbc_gpu_launch_config *config);
 int icbc_gpu_get_launch_config(int level, icbc_gpu_launch_config *config);

@@ -1,0 +1,9 @@
+// bc1_shares.h's rules as plain functions (built and called by tests/test_shares.py).
+#include "../icbc_gb300/csrc/bc1_shares.h"
+
+extern "C" {
+void batch(const int *levels, const int64_t *blocks, int n, int64_t warps, int level_kernels, int *sizes, int *ctas) {
+    const icbc_gpu::BatchShape s = icbc_gpu::batch_shape(levels, blocks, n, warps, level_kernels != 0);
+    for (int l = 0; l < 10; l++) sizes[l] = s.task_blocks[l], ctas[l] = s.cta_warps[l];
+}
+}
