@@ -128,7 +128,7 @@ inline cudaError_t launch_encode_batch(const GlobalTables *G, const ImageDesc *i
 // empty refinement slot) and lists the rest.  A grid stride over the first
 // ntasks tasks (`tasks`, or per-image offsets as for launch_encode_batch).
 cudaError_t launch_batch_trivial(const GlobalTables *G, const ImageDesc *images, const BatchTask *tasks,
-                                 const uint32_t *task_start, int n_images, int ntasks, BatchLists lists,
+                                 const uint32_t *task_start, int n_images, int ntasks, bool levels_8_9, BatchLists lists,
                                  const int64_t *refine_base, RefineSlot *slots, cudaStream_t stream, int sms);
 // Loads launch_batch_trivial's kernel (which otherwise loads on its first launch).
 void prepare_batch_trivial();

@@ -554,6 +554,8 @@ int icbc_gpu_batch_create(const icbc_gpu_image *images, int n_images, icbc_gpu_b
         levels.push_back(descs[i].level);
         counts.push_back(descs[i].nblocks);
     }
+    bool levels_8_9 = false;
+    for (int l : levels) levels_8_9 |= l >= 8;
     const BatchShape shape = batch_shape(levels.data(), counts.data(), (int)levels.size(),
                                          (int64_t)grid * kWarpsPerCta, byte_rows);
     for (int i : order) {
@@ -676,7 +678,7 @@ int icbc_gpu_batch_create(const icbc_gpu_image *images, int n_images, icbc_gpu_b
         if (e1 == cudaSuccess && B->d_list) {
             e1 = cudaMemsetAsync(B->d_listed, 0, sizeof(unsigned int) * n_images, cs);
             if (e1 == cudaSuccess)
-                e1 = launch_batch_trivial(G, B->d_images, B->d_tasks, nullptr, n_images, B->ntasks_listed, lists,
+                e1 = launch_batch_trivial(G, B->d_images, B->d_tasks, nullptr, n_images, B->ntasks_listed, levels_8_9, lists,
                                           B->d_refine_base, B->d_slots, cs, sm_count());
         }
         cudaError_t e2 = e1;

@@ -248,7 +248,7 @@ int launch_slot(icbc_gpu_server *S, Slot &slot) {
                             slot.stream);
         if (e == cudaSuccess) e = cudaMemsetAsync(slot.d_listed, 0, sizeof(unsigned int) * n, slot.stream);
         if (e == cudaSuccess)
-            e = launch_batch_trivial(S->G, slot.d_images, nullptr, slot.d_start, n, (int)listed_tasks, lists, nullptr, nullptr,
+            e = launch_batch_trivial(S->G, slot.d_images, nullptr, slot.d_start, n, (int)listed_tasks, true, lists, nullptr, nullptr,
                                      slot.stream, current_sm_count());
     }
     if (e == cudaSuccess) {
