@@ -1196,12 +1196,17 @@ __device__ __forceinline__ float encode_warp_ex(const WarpCtx &w, const Row &row
     // needs: 8, 12 (levels 2-5) or 16 entries (warp-uniform; levels 2-7, where
     // most blocks reduce to a few colours; at levels 8-9 the extra builds'
     // code cost 0.4%).  Each width is 10-20 KB of straight-line code, so the
-    // 12-wide build, whose warps are few at levels 6-7, and narrow ones for
-    // the rarer rebuild without black colours cost more instruction fetches
-    // than they saved: without them 4096 x 4096 at level 7 927 -> 906 us, the
-    // hard mixture at level 6 2058 -> 1962.
+    // 12-wide build, whose warps are few at levels 6-7, and from level 4 on
+    // narrow ones for the rarer rebuild without black colours (NARROW) cost
+    // more instruction fetches than they saved: without them 4096 x 4096 at
+    // level 7 927 -> 906 us, the hard mixture at level 6 2058 -> 1962.  At
+    // levels 2-3, and in the warp-wide kernels of byte rows at level 4, they
+    // pay: without / with, batches of 160,000 blocks at level 2 83 / 75 us, at
+    // level 3 80 / 73, 400,000 at level 4 149 / 134 (400,000 of the hard mixture
+    // 1271 / 1301).
     const int wmax = O::cluster && L <= 7 && !SIMD ? __reduce_max_sync(kFull, active ? count : 0) : 16;
     const int width = wmax <= 8 ? 8 : wmax <= 12 ? 12 : 16;
+    constexpr bool NARROW = L <= 3 || (L == 4 && NW == 1 && Row::kBytes);
     // Float rows at levels 8-9, where the search is nearly all of the work,
     // take the bounded arithmetic when the warp's colours allow it (the check
     // is 0.2% of the work; 1000 x 1000 with a weight plane at level 8 376 -> 319 us,
@@ -1266,7 +1271,9 @@ __device__ __forceinline__ float encode_warp_ex(const WarpCtx &w, const Row &row
                     // then build the table of the non-black ones.
                     bool ab;
                     reduce_level<L>(row, srow, ab);
-                    count3 = build_sat_inplace(srow, count, true);
+                    count3 = NARROW && width == 8    ? build_sat_inplace<8>(srow, count, true)
+                             : NARROW && width == 12 ? build_sat_inplace<12>(srow, count, true)
+                                                     : build_sat_inplace(srow, count, true);
                     if (SIMD) fill_sat_tail(srow, count3, p.simd_gather);
                     need3 = count3 > 0;
                 } else {
