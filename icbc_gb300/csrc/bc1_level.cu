@@ -205,7 +205,7 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32, 4) k_image_listed(const Glo
                                                                        EncodeParams p, const uint32_t *list,
                                                                        const unsigned int *listed, RefineSlot *st) {
     const int64_t n = *listed;
-    const int per_warp = balanced_share(n, (int64_t)gridDim.x * kWarpsPerCta, 32, least_per_warp(L));
+    const int per_warp = image_share(n, (int64_t)gridDim.x * kWarpsPerCta, L);
     const int64_t groups = (n + per_warp - 1) / per_warp;
     if ((int64_t)blockIdx.x * kWarpsPerCta >= groups) return;  // the whole CTA has no work
     extern __shared__ __align__(16) unsigned char smem[];
@@ -473,7 +473,8 @@ constexpr bool kCompact = Level<L>::cluster;
 // kBalancedRounds rounds gives each warp one group of a balanced size.
 constexpr int kBalancedRounds = 8;
 template <class K>
-static int grid_for(K kernel, int64_t n, int sms, size_t smem, int &resident, int *per_warp = nullptr) {
+static int grid_for(K kernel, int64_t n, int sms, size_t smem, int &resident, bool image = true,
+                    int *per_warp = nullptr) {
     const LaunchShape shape = launch_shape(L);
     if (!resident) {
         int per_sm = 0;
@@ -486,7 +487,8 @@ static int grid_for(K kernel, int64_t n, int sms, size_t smem, int &resident, in
     if (per_warp) {
         *per_warp = 32;
         if (L >= 2 && n < cap * kWarpsPerCta * 32 * kBalancedRounds) {
-            *per_warp = balanced_share(n, cap * kWarpsPerCta, 32, least_per_warp(L));
+            *per_warp = image ? image_share(n, cap * kWarpsPerCta, L)
+                              : balanced_share(n, cap * kWarpsPerCta, 32, least_per_warp(L));
             return (int)((n + (int64_t)*per_warp * kWarpsPerCta - 1) / ((int64_t)*per_warp * kWarpsPerCta));
         }
     }
@@ -519,7 +521,7 @@ static cudaError_t run(Kernel kernel, size_t smem, int &resident, int64_t n, int
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     int per_warp = 32;
-    const int grid = grid_for(kernel, n, sms, smem, resident, &per_warp);
+    const int grid = grid_for(kernel, n, sms, smem, resident, image != nullptr, &per_warp);
     if (!kDefer) {
         launch(grid, smem, per_warp, nullptr);
         return cudaGetLastError();

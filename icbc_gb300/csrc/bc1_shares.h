@@ -32,6 +32,16 @@ ICBC_HD constexpr int balanced_share(int64_t n, int64_t workers, int most, int l
 }
 ICBC_HD constexpr int least_per_warp(int level) { return level >= 4 ? 1 : 16; }
 
+// The share of an image's n blocks.  Below level 4 an image of more than one
+// round of the workers takes 32 a warp: its warps take much the same time
+// however few blocks they have, so even rounds only make more of them (levels
+// 2 / 3, even / 32, us: 1100 x 1100 with a weight plane 55 / 51 and 60 / 56,
+// 1448 x 1448 of the hard mixture 322 / 305 and 317 / 314).  Float blocks keep
+// even rounds (65,000 of the mixture at level 2 199, 218 with 32 a warp).
+ICBC_HD constexpr int image_share(int64_t n, int64_t workers, int level) {
+    return level < 4 && n > workers * 32 ? 32 : balanced_share(n, workers, 32, least_per_warp(level));
+}
+
 // How a batch is cut into tasks and launched, per level.
 //
 // A task is a warp's work, and its time grows with its blocks where the search

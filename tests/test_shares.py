@@ -1,5 +1,5 @@
 """CPU: the rules that share work out (icbc_gb300/csrc/bc1_shares.h): blocks
-per task of a batch."""
+per task of a batch, blocks per warp of an image."""
 import ctypes
 import os
 import random
@@ -23,6 +23,7 @@ def rules(tmp_path_factory):
     subprocess.run([cxx, "-O1", "-std=c++17", "-shared", "-fPIC", os.path.join(HERE, "shares_check.cpp"), "-o", out],
                    check=True)
     lib = ctypes.CDLL(out)
+    lib.image.argtypes = [ctypes.c_int64, ctypes.c_int64, ctypes.c_int]
     return lib
 
 
@@ -72,3 +73,17 @@ def test_light_levels_keep_whole_warps(rules):
             if sizes[7] < 32 and any(lv in (6, 7) for lv in levels):
                 lights32 = [32 if 2 <= lv <= 5 else s for lv, s in enumerate(sizes)]
                 assert tasks(levels, blocks, lights32) <= warps
+
+
+def test_image_share(rules):
+    """Below level 4 an image of more than a round takes whole warps; from level 4 on rounds are shared out evenly."""
+    for n in (1, 500, 20000, 58368, 58369, 75625, 116000, 500000):
+        for workers in (FLOAT_WARPS, BYTE_WARPS):
+            for level in range(2, 10):
+                share = rules.image(n, workers, level)
+                assert 1 <= share <= 32
+                if level < 4:
+                    assert share == 32 if n > 32 * workers else share >= 16
+                else:
+                    rounds = -(-n // (32 * workers))
+                    assert -(-n // share) <= rounds * workers
