@@ -558,12 +558,16 @@ static int g_resident_trivial = 0, g_resident_listed = 0, g_resident_listed8 = 0
 static int g_resident_batch8 = 0, g_resident_batch16 = 0;
 
 // The listed pass's CTA size at this level: the launch shape's, else the
-// level's default -- 16-warp CTAs from level 4 on, 4 at levels 2-3, whose
-// short lists gain nothing from CTA-wide searches.
+// level's default -- 4 warps at levels 2-3, whose short lists gain nothing from
+// CTA-wide searches, 8 at levels 4-5, 16 above.  Where few blocks are listed, a
+// 16-warp CTA has work for a few of its warps only: level 4 with 16 / 8 warps,
+// 1448 x 1448 60 / 55 us, one seventh of it textured 75 / 61 (4 warps 50), the
+// hard mixture 269 / 272; 4096 x 4096 203 / 200, 1794 / 1792; at levels 6-7 16 is
+// 2% faster on the mixture and as fast on the others.
 static int listed_cta_warps() {
     const int c = launch_shape(L).cta_warps;
     if (c == 4 || c == 8 || c == 16) return c;
-    return L >= 4 ? 16 : 4;
+    return L >= 6 ? 16 : L >= 4 ? 8 : 4;
 }
 
 // The CTA size for an image of `nblocks` blocks.  A CTA-wide pass shares the

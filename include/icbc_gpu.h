@@ -359,7 +359,7 @@ int icbc_gpu_compress_bc1_mips(const icbc_gpu_image *image, int32_t levels, void
  * takes 4); 0 = the level's default.  An image too small to give every
  * resident warp 32 blocks takes smaller shares whatever the shape.  Defaults:
  * 1 / persistent at levels 0-1, 2 / not persistent at levels 2-9, cta_warps
- * 16 from level 4 on (else 4), batch_cta_warps 4 or 8 by the batch's levels
+ * 4 at levels 2-3, 8 at 4-5 and 16 at 6-9, batch_cta_warps 4 or 8 by the batch's levels
  * and block counts.  Not for use while launches run or batches are created. */
 typedef struct icbc_gpu_launch_config {
     int32_t groups_per_warp;
