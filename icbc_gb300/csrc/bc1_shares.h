@@ -1,5 +1,6 @@
 // bc1_shares.h -- how work is shared out: blocks per warp or CTA, blocks per
-// task of a batch.  Plain arithmetic on counts, for host and device code alike.
+// task of a batch, bands of a host-buffer call.  Plain arithmetic on counts,
+// for host and device code alike.
 #pragma once
 
 #include <stdint.h>
@@ -107,6 +108,34 @@ inline BatchShape batch_shape(const int *levels, const int64_t *blocks, int n, i
     set(2, 5, fit(2, 5, 1, 32, 3 * warps / 8 - used), heavy_tasks > 0 || (mid_tasks > 0 && wide));
     set(0, 1, 32, false);
     return s;
+}
+
+// Bands that a host-buffer call cuts an image of `blocks` blocks into: enough
+// to overlap the upload, most of the light levels' call, with the encode, but
+// each large enough for the encoder, for which blocks count and not rows.  In
+// us, by bands: level 1, 16384 x 512 272 (1) 239 (2) 222 (5) 223 (8); 2048 x
+// 2048 155 (1) 128 (4) 140 (8); 1024 x 1024 60 (1) 58 (2) 65 (4).  Level 3, 4096
+// x 4096 508 (1) 438 (4) 423 (6).  Level 8, 2048 x 2048 897 (1) 849 (3) 876 (4);
+// 4096 x 4096 3343 / 3100 / 3093; level 9 3992 / 3777 / 3761.
+//
+// Levels 4-7 take bands that one CTA-wide pass takes whole (512 blocks an SM,
+// one_cta_pass) where that makes at most five: level 4, 2048 x 2048 194 (1) 193
+// (2) 204 (3) 177 (4); 2400 x 2400 239 (1) 216 (2) 237 (3) 213 (5).  Above, large
+// ones at levels 4-5, which list their blocks again (4096 x 4096 at level 5 603
+// (2) 553 (4) 529 (6)), and five at levels 6-7, each of which leaves its last
+// round's SMs to the next (level 6 823 (2) 756 (4) 728 (5) 742 (8)).
+inline int host_bands(int level, int64_t blocks, int sms) {
+    constexpr int64_t k = 1024;
+    const auto bands = [&](int64_t first, int64_t each, int most) {
+        const int64_t b = blocks / each;
+        return blocks < first ? 1 : b < 2 ? 2 : b < most ? (int)b : most;
+    };
+    if (level < 2) return bands(48 * k, 64 * k, 5);
+    if (level < 4) return blocks < 640 * k ? bands(80 * k, 64 * k, 4) : bands(0, 160 * k, 6);
+    if (level >= 8) return bands(96 * k, 80 * k, 4);
+    const int64_t whole = (blocks + 512 * (int64_t)sms - 1) / (512 * (int64_t)sms);
+    if (whole <= 5) return (int)whole;
+    return level >= 6 ? 5 : bands(0, 160 * k, 6);
 }
 
 }  // namespace icbc_gpu

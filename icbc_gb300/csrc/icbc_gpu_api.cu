@@ -890,22 +890,9 @@ int icbc_gpu_compress_bc1_image_host(const uint8_t *rgba, int32_t width, int32_t
     if (e == cudaSuccess && weight_mode == ICBC_GPU_WEIGHTS_PLANE)
         e = grow(reinterpret_cast<void **>(&H.d_plane), &H.plane_bytes, sizeof(float) * (size_t)width * height);
     if (e != cudaSuccess) return set_cuda_error(e);
-    // Bands of whole block rows (each band is an independent image whose
-    // last band alone meets the bottom edge), at most kLevelBands[level] of at
-    // least kBandRows[level] block rows each: enough to overlap the upload, which is
-    // most of the light levels' call, with the encode, but each large enough
-    // for the encoder (level 9's refinement queue wants many blocks per lane).
-    // In us, against bands half as high, 4 from level 4 on (2 at levels 8-9):
-    // 2048 x 2048 at level 4 208 / 259, level 8 916 / 969; 1024 x 1024 at level
-    // 5 107 / 160; 4096 x 4096 at level 8 3321 / 3415.  Up to level 7 a band
-    // leaves its last round's SMs to the next one (levels 6-7 at 4096 x 4096
-    // 786 / 1073, evenly shared rounds 839 / 1091; at level 8 evenly shared
-    // ones are 5% faster).
-    static const int kLevelBands[10] = {8, 8, 8, 8, 5, 4, 4, 4, 3, 3};
-    static const int kBandRows[10] = {128, 128, 128, 128, 200, 128, 128, 128, 170, 170};
-    const int lv = level < 0 ? 0 : level > 9 ? 9 : level;
-    const int bands = (int)std::max<int64_t>(1, std::min<int64_t>(std::min(kMaxBands, kLevelBands[lv]),
-                                                                  bh / kBandRows[lv]));
+    // Bands of whole block rows; each is an independent image whose last band
+    // alone meets the bottom edge.
+    const int bands = host_bands(level, nb, sm_count());
     const int64_t rows_per = (bh + bands - 1) / bands;
     int st = ICBC_GPU_OK;
     for (int i = 0; i < bands && st == ICBC_GPU_OK; i++) {

@@ -1,5 +1,5 @@
 """CPU: the rules that share work out (icbc_gb300/csrc/bc1_shares.h): blocks
-per task of a batch, blocks per warp of an image."""
+per task of a batch, blocks per warp of an image, bands of a host-buffer call."""
 import ctypes
 import os
 import random
@@ -23,6 +23,7 @@ def rules(tmp_path_factory):
     subprocess.run([cxx, "-O1", "-std=c++17", "-shared", "-fPIC", os.path.join(HERE, "shares_check.cpp"), "-o", out],
                    check=True)
     lib = ctypes.CDLL(out)
+    lib.bands.argtypes = [ctypes.c_int, ctypes.c_int64, ctypes.c_int]
     lib.image.argtypes = [ctypes.c_int64, ctypes.c_int64, ctypes.c_int]
     return lib
 
@@ -87,3 +88,18 @@ def test_image_share(rules):
                 else:
                     rounds = -(-n // (32 * workers))
                     assert -(-n // share) <= rounds * workers
+
+
+@pytest.mark.parametrize("level", range(10))
+def test_host_bands(rules, level):
+    """Bands follow the number of blocks, whatever the image's sides: a low, wide image is cut as a square one is."""
+    last = 1
+    for k in (1, 16, 47, 64, 95, 128, 156, 200, 256, 352, 512, 706, 1024, 4096):
+        bands = rules.bands(level, k * 1024, SMS)
+        assert 1 <= bands <= 8
+        if k <= 16:
+            assert bands == 1
+        if k >= 512:
+            assert bands >= 3  # the upload overlaps
+        last = bands
+    assert last >= 3
