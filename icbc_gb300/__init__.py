@@ -59,6 +59,11 @@ class LaunchConfig(ctypes.Structure):
                 ("batch_cta_warps", ctypes.c_int32)]
 
 
+class LaunchInfo(ctypes.Structure):
+    """struct icbc_gpu_launch_info."""
+    _fields_ = [("passes", ctypes.c_int32), ("cta_warps", ctypes.c_int32), ("shaped_ctas", ctypes.c_int32)]
+
+
 class ServerConfig(ctypes.Structure):
     """struct icbc_gpu_server_config."""
     _fields_ = [("hbm_budget_bytes", ctypes.c_int64), ("max_inflight", ctypes.c_int32),
@@ -144,6 +149,8 @@ def load(build_if_missing: bool = True):
             "icbc_gpu_compress_bc1_mips": (i32, [ctypes.POINTER(ImageDesc), i32, vp]),
             "icbc_gpu_set_launch_config": (i32, [i32, ctypes.POINTER(LaunchConfig)]),
             "icbc_gpu_get_launch_config": (i32, [i32, ctypes.POINTER(LaunchConfig)]),
+            "icbc_gpu_launch_plan": (i32, [i32, ctypes.c_int32, ctypes.c_int32, ctypes.c_int32,
+                                           ctypes.POINTER(LaunchInfo)]),
             "icbc_gpu_write_ktx": (i32, [ctypes.c_char_p, i32, i32, vp]),
             "icbc_gpu_compare_dds": (i32, [ctypes.c_char_p, i32, i32, vp]),
             "icbc_gpu_compress_bc1_images_noalloc": (i32, [ctypes.POINTER(ImageDesc), i32, vp]),
@@ -649,6 +656,15 @@ def set_launch_config(level: int, groups_per_warp: int, persistent: int, cta_war
     _check(load().icbc_gpu_set_launch_config(int(level), ctypes.byref(c)), "set_launch_config")
 
 
+def launch_plan(level: int, width: int, height: int, weight_mode: int = WEIGHTS_UNIFORM) -> tuple[int, int, int]:
+    """(passes, cta_warps, shaped_ctas): how compress_image launches an image
+    of this size under the level's launch shape (icbc_gpu_launch_plan)."""
+    c = LaunchInfo()
+    _check(load().icbc_gpu_launch_plan(int(level), int(width), int(height), int(weight_mode), ctypes.byref(c)),
+           "launch_plan")
+    return c.passes, c.cta_warps, c.shaped_ctas
+
+
 def get_batch_cta_warps(level: int) -> int:
     """The batched form's CTA size at a level (0: the default, 4 or 8 by the
     batch's levels and block counts)."""
@@ -701,7 +717,10 @@ def autotune(image, levels=range(10), candidates=TUNE_CANDIDATES, cta_candidates
     uint8 tensor (h, w, 4)) for each level with CUDA events and keeps the
     fastest (applied to the library when `apply`): first (groups_per_warp,
     persistent) over `candidates`, then, at levels 2-9, the listed pass's CTA
-    size over `cta_candidates`.  Returns {level: {"groups_per_warp",
+    size over `cta_candidates`.  Candidates that launch this image alike
+    (launch_plan) are timed once, and of such the shape in force, or else the
+    level's default, is kept: an image too small for a setting to reach its
+    launch says nothing about it.  Returns {level: {"groups_per_warp",
     "persistent", "cta_warps", "ms", "candidates": {...}}}.  With `path` the
     table is also written as JSON (load_tuning reads it)."""
     import json
@@ -712,7 +731,15 @@ def autotune(image, levels=range(10), candidates=TUNE_CANDIDATES, cta_candidates
     with torch.cuda.stream(stream):
         out = torch.zeros((nb, 8), dtype=torch.uint8, device=image.device)
 
-    def timed():
+    w, h = int(image.shape[1]), int(image.shape[0])
+
+    def timed(by_plan):
+        plan = launch_plan(lv, w, h, weight_mode)
+        if plan not in by_plan:
+            by_plan[plan] = _timed()
+        return by_plan[plan]
+
+    def _timed():
         with torch.cuda.stream(stream):
             compress_image(image, lv, decoder, color_weights, weight_mode, out=out, stream=stream)
             e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
@@ -726,20 +753,26 @@ def autotune(image, levels=range(10), candidates=TUNE_CANDIDATES, cta_candidates
     table = {}
     for lv in levels:
         before = get_launch_config(lv)
-        times = {}
+        times, by_plan = {}, {}
         for g, p in candidates:
             set_launch_config(lv, g, p, before[2])
-            times["%d/%d" % (g, p)] = timed()
+            times["%d/%d" % (g, p)] = timed(by_plan)
         best = min(times, key=times.get)
+        kept = "%d/%d" % before[:2]
+        if times.get(kept) == times[best]:
+            best = kept
         g, p = (int(x) for x in best.split("/"))
         cta = before[2]
         if lv >= 2 and cta_candidates:
             ctimes = {}
             for c in cta_candidates:
                 set_launch_config(lv, g, p, c)
-                ctimes[c] = timed()
+                ctimes[c] = timed(by_plan)
                 times["%d/%d/cta%d" % (g, p, c)] = ctimes[c]
             cta = min(ctimes, key=ctimes.get)
+            kept = before[2] or (4 if lv < 4 else 8 if lv < 6 else 16)
+            if ctimes.get(kept) == ctimes[cta]:
+                cta = kept
             best = "%d/%d/cta%d" % (g, p, cta)
         set_launch_config(lv, *((g, p, cta) if apply else before))
         table[int(lv)] = {"groups_per_warp": g, "persistent": p, "cta_warps": cta, "ms": times[best],

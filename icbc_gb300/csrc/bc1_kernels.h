@@ -46,6 +46,7 @@ struct alignas(16) BatchTask {
 using BlocksLauncher = cudaError_t (*)(const GlobalTables *, const BlocksSrc &, const EncodeParams &, void *, float *,
                                        int64_t, cudaStream_t, int);
 using ImageLauncher = cudaError_t (*)(const GlobalTables *, const ImageDesc &, const EncodeParams &, cudaStream_t, int);
+using ImagePlanner = icbc_gpu_launch_info (*)(const ImageDesc &, int);
 using ImageLauncherExt = cudaError_t (*)(const GlobalTables *, const ImageDesc &, const EncodeParams &, cudaStream_t,
                                          int, RefineSlot *, unsigned long long *);
 
@@ -54,7 +55,8 @@ using ImageLauncherExt = cudaError_t (*)(const GlobalTables *, const ImageDesc &
                                    int64_t, cudaStream_t, int);                                                  \
     cudaError_t launch_image_l##L(const GlobalTables *, const ImageDesc &, const EncodeParams &, cudaStream_t, int); \
     cudaError_t launch_image_ext_l##L(const GlobalTables *, const ImageDesc &, const EncodeParams &, cudaStream_t, int, \
-                                      RefineSlot *, unsigned long long *);
+                                      RefineSlot *, unsigned long long *);                                         \
+    icbc_gpu_launch_info image_plan_l##L(const ImageDesc &, int);
 ICBC_DECLARE_LEVEL(0)
 ICBC_DECLARE_LEVEL(1)
 ICBC_DECLARE_LEVEL(2)

@@ -478,6 +478,7 @@ static int grid_for(K kernel, int64_t n, int sms, size_t smem, int &resident, bo
     const LaunchShape shape = launch_shape(L);
     if (!resident) {
         int per_sm = 0;
+        if (smem) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kWarpsPerCta * 32, smem) != cudaSuccess ||
             per_sm < 1)
             per_sm = 1;
@@ -684,10 +685,15 @@ static cudaError_t launch_image_compacted(const GlobalTables *G, const ImageDesc
 // 6 27 / 41; level 8 30 / 43, 384 x 384 84 / 88, 512 x 512 115 / 105.
 static bool one_pass(int64_t nblocks, int sms) { return nblocks < (int64_t)sms * (L >= 4 ? 96 : 512); }
 
+// Whether launch_image_compacted's kernels take the image.
+static bool compacted(const ImageDesc &d, int sms) {
+    return kCompact && use_byte_rows(d) && d.nblocks < (int64_t(1) << 32) && !one_pass(d.nblocks, sms);
+}
+
 static cudaError_t launch_image(const GlobalTables *G, const ImageDesc &d, const EncodeParams &p, cudaStream_t stream,
                                 int sms, RefineSlot *ext_st, unsigned long long *ext_counter) {
     if constexpr (kCompact) {
-        if (use_byte_rows(d) && d.nblocks < (int64_t(1) << 32) && !one_pass(d.nblocks, sms))
+        if (compacted(d, sms))
             return launch_image_compacted(G, d, p, stream, sms, ext_st, ext_counter);
     }
     if constexpr (Level<L>::cluster) {
@@ -704,6 +710,26 @@ static cudaError_t launch_image(const GlobalTables *G, const ImageDesc &d, const
                    k_encode_image<L, kDefer><<<grid, kWarpsPerCta * 32, smem, stream>>>(G, d, p, per_warp, slots);
                },
                G, &d, nullptr, p, d.out, d.errors, ext_st, ext_counter);
+}
+
+// The kernels launch_image takes and what of the launch shape reaches them.
+icbc_gpu_launch_info ICBC_CAT(image_plan_l, ICBC_LEVEL)(const ImageDesc &d, int sms) {
+    int per_warp = 32;
+    if constexpr (kCompact) {
+        if (compacted(d, sms)) {
+            const int cta_warps = listed_cta_warps(d.nblocks, sms);
+            if (cta_warps != 4 && one_cta_pass(d.nblocks, sms)) return {1, cta_warps, 0};
+            return {2, cta_warps, grid_for(k_image_trivial<L>, d.nblocks, sms, 0, g_resident_trivial)};
+        }
+        if (use_byte_rows(d)) {
+            const int grid = grid_for(k_encode_image_bytes<L, kDefer>, d.nblocks, sms, smem_bytes_byte_rows(),
+                                      g_resident_bytes, true, &per_warp);
+            return {1, kWarpsPerCta, grid};
+        }
+    }
+    const int grid = grid_for(k_encode_image<L, kDefer>, d.nblocks, sms,
+                              L < 2 ? smem_bytes_image() : smem_bytes(Level<L>::cluster), g_resident_image, true, &per_warp);
+    return {1, kWarpsPerCta, grid};
 }
 
 cudaError_t ICBC_CAT(launch_blocks_l, ICBC_LEVEL)(const GlobalTables *G, const BlocksSrc &s, const EncodeParams &p,

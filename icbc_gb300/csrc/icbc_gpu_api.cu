@@ -158,6 +158,8 @@ const ImageLauncherExt kImageLaunchExt[10] = {launch_image_ext_l0, launch_image_
                                               launch_image_ext_l3, launch_image_ext_l4, launch_image_ext_l5,
                                               launch_image_ext_l6, launch_image_ext_l7, launch_image_ext_l8,
                                               launch_image_ext_l9};
+const ImagePlanner kImagePlan[10] = {image_plan_l0, image_plan_l1, image_plan_l2, image_plan_l3, image_plan_l4,
+                                     image_plan_l5, image_plan_l6, image_plan_l7, image_plan_l8, image_plan_l9};
 const BatchLevelLauncher kBatchLevelLaunch[10] = {launch_batch_level_l0, launch_batch_level_l1, launch_batch_level_l2,
                                                   launch_batch_level_l3, launch_batch_level_l4, launch_batch_level_l5,
                                                   launch_batch_level_l6, launch_batch_level_l7, launch_batch_level_l8,
@@ -394,6 +396,23 @@ int icbc_gpu_set_launch_config(int level, const icbc_gpu_launch_config *config) 
 int icbc_gpu_get_launch_config(int level, icbc_gpu_launch_config *config) {
     if (level < 0 || level > 9 || !config) return ICBC_GPU_ERR_INVALID_ARGUMENT;
     *config = g_launch[level];
+    return ICBC_GPU_OK;
+}
+
+int icbc_gpu_launch_plan(int level, int32_t width, int32_t height, int32_t weight_mode, icbc_gpu_launch_info *info) {
+    if (level < 0 || level > 9 || width < 1 || height < 1 || weight_mode < 0 || weight_mode > 2 || !info)
+        return ICBC_GPU_ERR_INVALID_ARGUMENT;
+    int devices = 0;
+    const cudaError_t e = cudaGetDeviceCount(&devices);
+    if (e != cudaSuccess) return set_cuda_error(e);
+    ImageDesc d{};
+    d.level = level;
+    d.weight_mode = weight_mode;
+    d.width = width;
+    d.height = height;
+    d.bw = (int)(((int64_t)width + 3) / 4);
+    d.nblocks = d.bw * (((int64_t)height + 3) / 4);
+    *info = kImagePlan[level](d, sm_count());
     return ICBC_GPU_OK;
 }
 

@@ -354,13 +354,24 @@ int icbc_gpu_compress_bc1_mips(const icbc_gpu_image *image, int32_t levels, void
  * of that level, read when a batch is created): 4 = CTAs of 4 warps,
  * each warp searching its own 32 blocks' cluster combinations; 8 or 16 =
  * CTAs of that many warps moving through the encoder's stages together, the
- * combinations of all the CTA's blocks searched by all its threads (an image
- * of fewer than 512 blocks an SM takes 8 instead of 16, one of fewer than 96
- * takes 4); 0 = the level's default.  An image too small to give every
- * resident warp 32 blocks takes smaller shares whatever the shape.  Defaults:
- * 1 / persistent at levels 0-1, 2 / not persistent at levels 2-9, cta_warps
- * 4 at levels 2-3, 8 at 4-5 and 16 at 6-9, batch_cta_warps 4 or 8 by the batch's levels
- * and block counts.  Not for use while launches run or batches are created. */
+ * combinations of all the CTA's blocks searched by all its threads; 0 = the
+ * level's default.
+ * Small images decide part of their launch by their size, whatever the
+ * shape; icbc_gpu_launch_plan says how an image is launched:
+ *   - RGBA8 images without a weight plane at levels 2-9 take one kernel of
+ *     4-warp CTAs, and cta_warps does not apply, below 96 blocks an SM (512 at
+ *     levels 2-3); from there to 512 blocks an SM 16 means 8; and at levels
+ *     4-7, up to 512 (levels 4-5) or 900 blocks an SM, CTAs of 8 or 16 warps
+ *     take the whole image without a first pass.
+ *   - groups_per_warp and persistent shape the first pass of the images in two
+ *     passes and every launch at levels 0-1.  The other kernels of levels 2-9
+ *     (these small images, images with a weight plane, float blocks) follow
+ *     them only from eight rounds of 32 blocks for every resident warp on;
+ *     smaller work is shared out evenly.
+ * Defaults: 1 / persistent at levels 0-1, 2 / not persistent at levels 2-9;
+ * cta_warps 4 at levels 2-3, 8 at 4-5 and 16 at 6-9; batch_cta_warps 4 or 8
+ * by the batch's levels and block counts.  Not for use while launches run or
+ * batches are created. */
 typedef struct icbc_gpu_launch_config {
     int32_t groups_per_warp;
     int32_t persistent;
@@ -369,6 +380,19 @@ typedef struct icbc_gpu_launch_config {
 } icbc_gpu_launch_config;
 int icbc_gpu_set_launch_config(int level, const icbc_gpu_launch_config *config);
 int icbc_gpu_get_launch_config(int level, icbc_gpu_launch_config *config);
+
+/* How icbc_gpu_compress_bc1_image launches an image of this size on the
+ * current device under the level's present launch shape: two shapes with the
+ * same plan make the same launches.  passes: kernels that encode blocks (2:
+ * a first pass finishes the blocks of 0 or 1 colours and lists the others);
+ * cta_warps: warps a CTA of the last of them; shaped_ctas: CTAs of the kernel
+ * that groups_per_warp and persistent may shape (0: none). */
+typedef struct icbc_gpu_launch_info {
+    int32_t passes;
+    int32_t cta_warps;
+    int32_t shaped_ctas;
+} icbc_gpu_launch_info;
+int icbc_gpu_launch_plan(int level, int32_t width, int32_t height, int32_t weight_mode, icbc_gpu_launch_info *info);
 
 /* Number of SMs of the current device (for sizing host-side work). */
 int icbc_gpu_sm_count(void);
