@@ -79,11 +79,13 @@ def launches_per_level(level: int) -> int:
 
 def level_kernels(level: int) -> str:
     """The launches of one level call on the RGBA8 image with alpha weights
-    (the default shapes: a CTA-wide listed pass from level 4 on)."""
+    (the default shapes: a listed pass of 8-warp CTAs at levels 4-5, 16-warp
+    ones from level 6 on)."""
     if level < 2:
         return "k_encode_image<%d>" % level
-    listed = "k_image_listed<%d>" % level if level < 4 else "k_image_listed_cta<%d, %d, 16>" % (level, level == 9)
-    return "k_image_trivial<%d> + %s" % (level, listed) + (" + k_refine<1>" if level == 9 else "")
+    listed = "k_image_listed<%d>" % level if level < 4 else "k_image_listed_cta<%d, %d, %d>" % (
+        level, level == 9, 8 if level < 6 else 16)
+    return "k_image_trivial<%d> + %s" % (level, listed) + (" + k_refine<1, 4>" if level == 9 else "")
 
 
 def algorithmic_ops(stats: dict, level: int) -> float:

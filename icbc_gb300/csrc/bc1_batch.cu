@@ -15,9 +15,9 @@ namespace icbc_gpu {
 constexpr bool kBytes = ICBC_BATCH_BYTES != 0;
 
 // Persistent batched encoder over mixed levels and decoders: every warp
-// takes the next task (32 blocks of one image) from an atomic counter until
-// the queue is empty (run_batch); tasks are ordered most expensive level
-// first by the planner.
+// takes the next task (up to 32 blocks of one image) from an atomic counter
+// until the queue is empty (run_batch); tasks are ordered most expensive
+// level first by the planner.
 template <bool BYTES>
 __global__ void __launch_bounds__(kWarpsPerCta * 32, BYTES ? 4 : 1)
     k_encode_batch(const GlobalTables *G, const ImageDesc *images, const BatchTask *tasks, const uint32_t *task_start,
@@ -29,8 +29,8 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32, BYTES ? 4 : 1)
 
 #if ICBC_BATCH_BYTES
 // First pass of a two-pass batch: every warp takes tasks of the listed
-// images (list_base >= 0, levels 2..9) in a grid stride and follows
-// reduce_colors (icbc.h:1683-1728) in registers for its blocks, as
+// images (list_base >= 0, levels 2..9) in a grid stride and tells its blocks
+// of 0 or 1 reduced colours (icbc.h:1683-1728) in registers, as
 // k_image_trivial does for one image: a block of 0 or 1 reduced colours is
 // finished here (icbc.h:3752-3764; at level 9 with an empty refinement slot),
 // any other goes to its image's list with one atomic per warp.  Only the u8

@@ -13,8 +13,8 @@ __device__ __forceinline__ BatchTask load_task(const BatchTask *t) {
 }
 
 // Task t of a batch: an entry of the explicit list, or -- without one, tasks
-// of 32 blocks -- found from per-image offsets: task t belongs to the last image whose first
-// task (`task_start[i]`, n_images + 1 entries) is <= t.
+// of 32 blocks -- found from per-image offsets: task t belongs to the last
+// image whose first task (`task_start[i]`, n_images + 1 entries) is <= t.
 __device__ __forceinline__ BatchTask batch_task(const BatchTask *tasks, const uint32_t *task_start, int n_images,
                                                 int t) {
     if (tasks) return load_task(tasks + t);

@@ -69,9 +69,6 @@ ICBC_DECLARE_LEVEL(8)
 ICBC_DECLARE_LEVEL(9)
 #undef ICBC_DECLARE_LEVEL
 
-// With refine_base (one entry per image; -1: refine inline) a level-9 image's
-// refinement is deferred: block b's RefineSlot goes to slots[refine_base[i] + b]
-// and launch_refine_batch finishes it.  NULL refine_base: all inline.
 // The blocks the first pass of a two-pass batch left to the second: image
 // i's are list[list_base[i] .. list_base[i] + listed[i]) (list_base[i] < 0:
 // the image is not in two passes and its tasks cover its blocks in order).
@@ -102,6 +99,9 @@ ICBC_DECLARE_BATCH_LEVEL(8)
 ICBC_DECLARE_BATCH_LEVEL(9)
 #undef ICBC_DECLARE_BATCH_LEVEL
 
+// With refine_base (one entry per image; -1: refine inline) a level-9 image's
+// refinement is deferred: block b's RefineSlot goes to slots[refine_base[i] + b]
+// and launch_refine_batch finishes it.  NULL refine_base: all inline.
 // byte_rows: the kernel with byte texel rows (no image of the batch has a
 // weight plane), four CTAs per SM; else float rows.  With lists.list, the
 // tasks of listed images take their blocks from the lists.

@@ -150,13 +150,13 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32, 4) k_encode_image_bytes(con
 // listed blocks per warp.  Each block's computation is the single-pass one
 // (pass 2 reduces again).  Levels 2-4 take half the time, levels 5-8 2-25%
 // less.
-// Pass 1 needs only to tell blocks of 0 or 1 reduced colours from the rest,
-// so it follows reduce_colors (icbc.h:1683-1728) only while one colour has
-// been kept: the texels and the running colour stay in registers (a ByteRow
-// over a register array, every index known at compile time), and a block
-// is listed as soon as a second colour appears.  For the blocks it finishes
-// the arithmetic is reduce_colors' (every texel merged into the first
-// colour).  Shared memory holds only the i / 255 table; six CTAs per SM
+// Pass 1 needs only to tell blocks of 0 or 1 reduced colours from the rest.
+// Levels 8-9 compare bytes (one_byte_colour).  Levels 2-7 follow reduce_colors
+// (icbc.h:1683-1728) only while one colour has been kept: the texels and the
+// running colour stay in registers (a ByteRow over a register array, every
+// index known at compile time), and a block is listed as soon as a second
+// colour appears.  For the blocks it finishes the arithmetic is reduce_colors'
+// (every texel merged into the first colour).  Shared memory holds only the i / 255 table; six CTAs per SM
 // (80 registers) beat both four (126 registers) and eight (more spills).
 template <int L>
 __global__ void __launch_bounds__(kWarpsPerCta * 32, 6) k_image_trivial(const GlobalTables *G, ImageDesc d, EncodeParams p,
@@ -238,10 +238,6 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32, 4) k_image_listed(const Glo
     }
 }
 
-// The batched form's kernel for this level's tasks of a byte-row batch:
-// run_batch with the level fixed, so the kernel holds one level's code as the
-// plain kernels do (the all-levels kernel stalls about twice as often on
-// instruction fetch for the same blocks).
 // k_image_listed with the CTA as the unit: NW warps take 32 * NW listed
 // blocks at a time and move through the encoder's stages together -- colour
 // reduction and summed-area tables one block per lane, then the cluster
@@ -453,6 +449,10 @@ __global__ void __launch_bounds__(NW * 32, 512 / (NW * 32))
     }
 }
 
+// The batched form's kernel for this level's tasks of a byte-row batch:
+// run_batch with the level fixed, so the kernel holds one level's code as the
+// plain kernels do (the all-levels kernel stalls about twice as often on
+// instruction fetch for the same blocks).
 template <int LV>
 __global__ void __launch_bounds__(kWarpsPerCta * 32, 4)
     k_batch_level(const GlobalTables *G, const ImageDesc *images, const BatchTask *tasks, int task0, int ntasks,

@@ -316,7 +316,7 @@ static cudaError_t refine_launch(const GlobalTables *G, const ImageDesc &d, cons
 // of the hard mixture 147 / 166 / 196, 10,000 215 / 203 / 235, 40,000 539 /
 // 376 / 402, 200,000 1797 / 1203 / 1171; 1024 x 1024 328 / 314 / 323, 4096 x
 // 4096 3920 / 3800 / 3773; a block a lane one step at a time: 133 us for 64 x
-// 64's pass alone).
+// 64's pass alone).  n counts slots, with something to refine or not.
 template <int MODE>
 static cudaError_t refine_pass(const GlobalTables *G, const ImageDesc &d, const BlocksSrc &s, const EncodeParams &p,
                                uint2 *out, float *errors, const RefineSlot *st, int64_t n, unsigned long long *counter,
