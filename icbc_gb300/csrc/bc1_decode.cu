@@ -12,9 +12,10 @@ constexpr unsigned kFullWarp = 0xffffffffu;
 // are then moved a block row (16 bytes) a lane, 8 blocks at a time, with the
 // block's palette and indices by shuffle, so that every load and store of the
 // warp covers 512 consecutive bytes.  With a block a lane each access touched
-// 32 half sectors 64 bytes apart: 2^22 blocks took 70 us to decode (4.3 TB/s)
-// and 78 to evaluate (4.1), now 48 (6.3) and 60 (5.3); 2^20 blocks 23 and 27,
-// now 17 and 21.  Bound by DRAM, evaluate by its shuffles and selects too.
+// 32 half sectors 64 bytes apart: 2^22 blocks took 68 us to decode (4.4 TB/s)
+// and 74 to evaluate (4.3), now 47 (6.5) and 51 (6.3); both on 2^20 blocks, one
+// after the other, 45 and now 33-34.  Bound by DRAM, evaluate by its shuffles
+// and selects too.
 //
 // Row `lane & 3` of the block that lane `src` holds: its 4 texels.
 __device__ __forceinline__ uint4 block_row(const uint32_t pk[4], uint32_t indices, int src) {

@@ -400,7 +400,6 @@ __device__ __forceinline__ bool optimize_end_points4(const Row &row, uint32_t in
 // `colors`: the reduced colours in a SAT row (SatColors) or a texel row.
 struct SatColors {
     static constexpr bool kBounded = false;
-    static constexpr int kBoxUnroll = 4;
     const float *p;
     __device__ __forceinline__ V3 color(int i) const { return xyz(ld4(p + 4 * i)); }
 };
@@ -409,7 +408,7 @@ template <class C>
 __device__ __forceinline__ void box_fit(const C &colors, int count, V3 &c0, V3 &c1) {
     c0 = v3(0.0f, 0.0f, 0.0f);
     c1 = v3(1.0f, 1.0f, 1.0f);
-#pragma unroll C::kBoxUnroll
+#pragma unroll 4
     for (int i = 0; i < count; i++) {
         const V3 c = colors.color(i);
         if (C::kBounded) {  // no NaN and no -0: the reference's max and min are fmaxf and fminf
@@ -427,7 +426,7 @@ __device__ __forceinline__ void box_fit(const C &colors, int count, V3 &c0, V3 &
     c1 = saturate(c1 + inset);
     const V3 center = (c0 + c1) * 0.5f;
     float cov_xz = 0.0f, cov_yz = 0.0f;
-#pragma unroll C::kBoxUnroll
+#pragma unroll 4
     for (int i = 0; i < count; i++) {
         const V3 t = colors.color(i) - center;
         cov_xz += t.x * t.z;
@@ -474,11 +473,11 @@ __device__ __forceinline__ uint32_t index_generic(V3 color, V3 cw, V3 p0, V3 p1,
 }
 
 // Generic nearest-of-four indices (compute_indices, icbc.h:3179-3235).
-template <int UNROLL = 1, class Row>
+template <class Row>
 __device__ __forceinline__ uint32_t indices_generic(const Row &row, V3 cw, const PalF &pal) {
     const V3 p0 = pal.c[0] * cw, p1 = pal.c[1] * cw, p2 = pal.c[2] * cw, p3 = pal.c[3] * cw;
     uint32_t out = 0;
-#pragma unroll UNROLL
+#pragma unroll 1
     for (int t = 0; t < 16; t++) out |= index_generic(row.color(t), cw, p0, p1, p2, p3) << (2 * t);
     return out;
 }

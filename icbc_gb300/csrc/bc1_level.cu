@@ -462,7 +462,6 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32, 4)
 }
 
 constexpr int L = ICBC_LEVEL;
-constexpr bool kCompact = Level<L>::cluster;
 
 // CTAs for n blocks and the blocks a warp takes at a time.  An image of many
 // rounds takes the level's launch shape: every warp takes groups_per_warp
@@ -549,14 +548,17 @@ static cudaError_t run(Kernel kernel, size_t smem, int &resident, int64_t n, int
 }
 
 // Resident CTAs per SM of each kernel (persistent launch shapes), found once.
-static int g_resident_blocks = 0, g_resident_image = 0, g_resident_bytes = 0;
+static int g_resident_blocks = 0, g_resident_image = 0;
+
+#if ICBC_LEVEL >= 2  // the cluster-fit levels, up to `#endif`
+static_assert(Level<L>::cluster, "");
 
 // Byte rows apply to the cluster-fit levels and to RGBA8 weights (uniform or
 // alpha); weight planes need float rows.
-static bool use_byte_rows(const ImageDesc &d) { return Level<L>::cluster && d.weight_mode != ICBC_GPU_WEIGHTS_PLANE; }
+static bool use_byte_rows(const ImageDesc &d) { return d.weight_mode != ICBC_GPU_WEIGHTS_PLANE; }
 
-static int g_resident_trivial = 0, g_resident_listed = 0, g_resident_listed8 = 0, g_resident_listed16 = 0;
-static int g_resident_batch8 = 0, g_resident_batch16 = 0;
+static int g_resident_bytes = 0, g_resident_trivial = 0, g_resident_listed = 0, g_resident_listed8 = 0;
+static int g_resident_listed16 = 0, g_resident_batch8 = 0, g_resident_batch16 = 0;
 
 // The listed pass's CTA size at this level: the launch shape's, else the
 // level's default -- 4 warps at levels 2-3, whose short lists gain nothing from
@@ -618,10 +620,10 @@ static cudaError_t listed_attributes(K kernel, int warps, size_t smem, int *resi
     return e;
 }
 
-// The passes of kCompact levels -- the CTA-wide one alone for smaller images
-// (one_cta_pass) -- with the list (and at level 9 the
-// refinement hand-over, unless the caller gives one) in stream-ordered
-// scratch; level 9 then runs its refinement pass over every block.
+// The two passes -- the CTA-wide one alone for smaller images (one_cta_pass) --
+// with the list (and at level 9 the refinement hand-over, unless the caller
+// gives one) in stream-ordered scratch; level 9 then runs its refinement pass
+// over every block.
 static cudaError_t launch_image_compacted(const GlobalTables *G, const ImageDesc &d, const EncodeParams &p,
                                           cudaStream_t stream, int sms, RefineSlot *ext_st,
                                           unsigned long long *ext_counter) {
@@ -687,24 +689,21 @@ static bool one_pass(int64_t nblocks, int sms) { return nblocks < (int64_t)sms *
 
 // Whether launch_image_compacted's kernels take the image.
 static bool compacted(const ImageDesc &d, int sms) {
-    return kCompact && use_byte_rows(d) && d.nblocks < (int64_t(1) << 32) && !one_pass(d.nblocks, sms);
+    return use_byte_rows(d) && d.nblocks < (int64_t(1) << 32) && !one_pass(d.nblocks, sms);
 }
+#endif
 
 static cudaError_t launch_image(const GlobalTables *G, const ImageDesc &d, const EncodeParams &p, cudaStream_t stream,
                                 int sms, RefineSlot *ext_st, unsigned long long *ext_counter) {
-    if constexpr (kCompact) {
-        if (compacted(d, sms))
-            return launch_image_compacted(G, d, p, stream, sms, ext_st, ext_counter);
-    }
-    if constexpr (Level<L>::cluster) {
-        if (use_byte_rows(d))
-            return run(k_encode_image_bytes<L, kDefer>, smem_bytes_byte_rows(), g_resident_bytes, d.nblocks, sms,
-                       stream,
-                       [&](int grid, size_t smem, int per_warp, RefineSlot *slots) {
-                           k_encode_image_bytes<L, kDefer><<<grid, kWarpsPerCta * 32, smem, stream>>>(G, d, p, per_warp, slots);
-                       },
-                       G, &d, nullptr, p, d.out, d.errors, ext_st, ext_counter);
-    }
+#if ICBC_LEVEL >= 2
+    if (compacted(d, sms)) return launch_image_compacted(G, d, p, stream, sms, ext_st, ext_counter);
+    if (use_byte_rows(d))
+        return run(k_encode_image_bytes<L, kDefer>, smem_bytes_byte_rows(), g_resident_bytes, d.nblocks, sms, stream,
+                   [&](int grid, size_t smem, int per_warp, RefineSlot *slots) {
+                       k_encode_image_bytes<L, kDefer><<<grid, kWarpsPerCta * 32, smem, stream>>>(G, d, p, per_warp, slots);
+                   },
+                   G, &d, nullptr, p, d.out, d.errors, ext_st, ext_counter);
+#endif
     return run(k_encode_image<L, kDefer>, L < 2 ? smem_bytes_image() : smem_bytes(Level<L>::cluster), g_resident_image, d.nblocks, sms, stream,
                [&](int grid, size_t smem, int per_warp, RefineSlot *slots) {
                    k_encode_image<L, kDefer><<<grid, kWarpsPerCta * 32, smem, stream>>>(G, d, p, per_warp, slots);
@@ -715,18 +714,16 @@ static cudaError_t launch_image(const GlobalTables *G, const ImageDesc &d, const
 // The kernels launch_image takes and what of the launch shape reaches them.
 icbc_gpu_launch_info ICBC_CAT(image_plan_l, ICBC_LEVEL)(const ImageDesc &d, int sms) {
     int per_warp = 32;
-    if constexpr (kCompact) {
-        if (compacted(d, sms)) {
-            const int cta_warps = listed_cta_warps(d.nblocks, sms);
-            if (cta_warps != 4 && one_cta_pass(d.nblocks, sms)) return {1, cta_warps, 0};
-            return {2, cta_warps, grid_for(k_image_trivial<L>, d.nblocks, sms, 0, g_resident_trivial)};
-        }
-        if (use_byte_rows(d)) {
-            const int grid = grid_for(k_encode_image_bytes<L, kDefer>, d.nblocks, sms, smem_bytes_byte_rows(),
-                                      g_resident_bytes, true, &per_warp);
-            return {1, kWarpsPerCta, grid};
-        }
+#if ICBC_LEVEL >= 2
+    if (compacted(d, sms)) {
+        const int cta_warps = listed_cta_warps(d.nblocks, sms);
+        if (cta_warps != 4 && one_cta_pass(d.nblocks, sms)) return {1, cta_warps, 0};
+        return {2, cta_warps, grid_for(k_image_trivial<L>, d.nblocks, sms, 0, g_resident_trivial)};
     }
+    if (use_byte_rows(d))
+        return {1, kWarpsPerCta, grid_for(k_encode_image_bytes<L, kDefer>, d.nblocks, sms, smem_bytes_byte_rows(),
+                                          g_resident_bytes, true, &per_warp)};
+#endif
     const int grid = grid_for(k_encode_image<L, kDefer>, d.nblocks, sms,
                               L < 2 ? smem_bytes_image() : smem_bytes(Level<L>::cluster), g_resident_image, true, &per_warp);
     return {1, kWarpsPerCta, grid};
@@ -746,8 +743,9 @@ cudaError_t ICBC_CAT(launch_batch_level_l, ICBC_LEVEL)(const GlobalTables *G, co
                                                         const BatchTask *tasks, int task0, int ntasks, int planned_warps,
                                                         int *counter, cudaStream_t stream, int grid, const int64_t *refine_base,
                                                         RefineSlot *slots, BatchLists lists) {
+#if ICBC_LEVEL >= 2
     // `grid` counts 4-warp CTAs; a CTA-wide kernel gets as many warps in all.
-    const int cta_warps = Level<L>::cluster && (L < 9 || refine_base) ? batch_cta_warps(planned_warps) : 4;
+    const int cta_warps = L < 9 || refine_base ? batch_cta_warps(planned_warps) : 4;
     if (cta_warps != 4) {
         const size_t smem = cta_warps == 16 ? batch_smem_bytes<16>() : batch_smem_bytes<8>();
         int *resident = cta_warps == 16 ? &g_resident_batch16 : &g_resident_batch8;
@@ -764,6 +762,7 @@ cudaError_t ICBC_CAT(launch_batch_level_l, ICBC_LEVEL)(const GlobalTables *G, co
                                                                      refine_base, slots, lists);
         return cudaGetLastError();
     }
+#endif
     const size_t smem = smem_bytes_byte_rows();
     cudaError_t e = cudaFuncSetAttribute(k_batch_level<L>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
